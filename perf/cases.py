@@ -13,7 +13,7 @@ outputs from direct summation in 64 bits.
 A pass starts from host arrays and ends with host arrays, as the solver's
 preprocess / solve / postprocess boundary does; from 1,000,000 particles on
 they are pinned buffers (upload_ptr / download_ptr), as bench.py's end-to-end
-measurement has them. The library's shipped tuning cache is in effect, as in
+measurement has them (a batch's inputs always). The library's shipped tuning cache is in effect, as in
 bench.py.
 """
 import math
@@ -50,7 +50,7 @@ def listed():
         # The reference's CPU-runnable configuration, ten RK4 steps in double precision as the reference runs them.
         _step("step_16k_fp64", "plummer", 16384, 4, 32, 0.01, 1e-3, 10, "fp64"),
         # An ordinary mixed-precision run at the library's default M2L split, ragged size.
-        _step("step_100k_mixed", "plummer", 100003, 8, 64, 0.005, 5e-4, 2, "mixed"),
+        _step("step_100k_mixed", "plummer", 100003, 8, 64, 0.005, 5e-4, 4, "mixed"),
         # Forces and potentials of an ordinary system in double precision (energy diagnostics).
         {"name": "accel_phi_131k_fp64", "kind": "accel", "model": "plummer", "n": 131071, "p": 8, "s": 64, "eps": 0.005,
          "precision": "fp64", "split": "tf32", "potential": True},
@@ -60,16 +60,16 @@ def listed():
         {"name": "direct_4k_of_262k", "kind": "direct", "model": "plummer", "n": 262144, "targets": 4096, "p": 8, "s": 64,
          "eps": 0.005, "precision": "mixed", "split": "bf16"},
         # The plain-at-scale unit cube, small leaves.
-        _step("step_cube_1m_bf16", "cube", 1048576, 6, 64, 1e-3, 1e-4, 1, "mixed", "bf16"),
+        _step("step_cube_1m_bf16", "cube", 1048576, 6, 64, 1e-3, 1e-4, 4, "mixed", "bf16"),
         # The accurate mode (softened far field) at its order, a size off the powers of two.
-        _step("step_accurate_1m", "plummer", 1000003, 10, 64, 0.005, 5e-4, 1, "mixed", "tf32", "accurate"),
-        # The headline: one step of the 4M Plummer sphere.
-        _step("step_plummer_4m_bf16", "plummer", 4194304, 8, 64, 0.005, 5e-4, 1, "mixed", "bf16"),
+        _step("step_accurate_1m", "plummer", 1000003, 10, 64, 0.005, 5e-4, 2, "mixed", "tf32", "accurate"),
+        # The headline: two steps of the 4M Plummer sphere.
+        _step("step_plummer_4m_bf16", "plummer", 4194304, 8, 64, 0.005, 5e-4, 2, "mixed", "bf16"),
         # Many independent systems of uneven size advanced together.
         {"name": "batch_512_bf16", "kind": "batch", "model": "plummer", "systems": 512, "n_lo": 1024, "n_hi": 65536, "p": 6,
-         "s": 64, "eps": 0.01, "dt": 5e-4, "steps": 1, "precision": "mixed", "split": "bf16"},
+         "s": 64, "eps": 0.01, "dt": 5e-4, "steps": 2, "precision": "mixed", "split": "bf16"},
         # The largest: the adaptive-depth stress workload.
-        _step("step_clusters_16m_bf16", "clusters", 16777216, 8, 64, 1e-4, 1e-4, 1, "mixed", "bf16"),
+        _step("step_clusters_16m_bf16", "clusters", 16777216, 8, 64, 1e-4, 1e-4, 2, "mixed", "bf16"),
     ]
 
 
@@ -94,9 +94,9 @@ def draw(rng):
     if family == "batch":
         lo = rng.choice([500, 1024, 2000])
         return {"kind": "batch", "model": "plummer", "systems": _log_int(rng, 8, 512), "n_lo": lo, "n_hi": rng.choice([8000, 30000, 65536]),
-                "p": rng.choice([4, 6, 8]), "s": rng.choice([32, 64]), "eps": 0.01, "dt": 5e-4, "steps": 1, "precision": "mixed",
+                "p": rng.choice([4, 6, 8]), "s": rng.choice([32, 64]), "eps": 0.01, "dt": 5e-4, "steps": 2, "precision": "mixed",
                 "split": rng.choice(["bf16", "bf16", "tf32"])}
-    c = _step("", "plummer", 0, 8, 64, eps, 5e-4, 1, "mixed")
+    c = _step("", "plummer", 0, 8, 64, eps, 5e-4, 2, "mixed")
     del c["name"]
     if family == "fp64":
         c.update(model=rng.choice(["plummer", "cube"]), n=_log_int(rng, 1000, 200000), p=rng.choice([4, 6, 7, 8]), s=rng.choice([32, 64]),
@@ -166,14 +166,15 @@ def _particles(case, seed):
     return x, v
 
 
-def _sizes(case, seed):
-    rng = np.random.default_rng([int(seed) & 0x7FFFFFFF, 7])
-    return rng.integers(case["n_lo"], case["n_hi"] + 1, case["systems"])
+def _sizes(case):
+    rng = np.random.default_rng([case["systems"], case["n_lo"], case["n_hi"]])
+    lo, hi = math.log(case["n_lo"]), math.log(case["n_hi"])  # uniform in the logarithm, as the batching workload
+    return np.exp(rng.uniform(lo, hi, case["systems"])).round().astype(np.int64)
 
 
 def _batch_particles(case, seed):
     """Every system a Plummer sphere of mass 1 scaled to a radius uniform in [0.5, 2]."""
-    g, sizes = _gen(seed), _sizes(case, seed)
+    g, sizes = _gen(seed), _sizes(case)
     x, v = _plummer(int(sizes.sum()), g)
     of = torch.repeat_interleave(torch.arange(len(sizes), device="cuda"), torch.from_numpy(sizes).cuda())
     r = (0.5 + 1.5 * _rand(g, len(sizes)))[of][:, None]
@@ -190,7 +191,7 @@ def prepare(case, seed):
         sizes, x, v = _batch_particles(case, seed)
         state["batch"] = vipp_gb300.Batch(sizes, p=case["p"], s=case["s"], eps=case["eps"], masses=1.0 / sizes,
                                           precision=case["precision"], flags=_flags(case))
-        state["x"], state["v"] = x.cpu().numpy(), v.cpu().numpy()
+        state["x"], state["v"] = (torch.empty(x.shape, dtype=x.dtype, pin_memory=True).copy_(q).numpy() for q in (x, v))
         return state
     x, v = _particles(case, seed)
     n = case["n"]
@@ -249,7 +250,7 @@ def work(case):
     """
     if case["kind"] == "direct":
         return {"bytes": 24.0 * case["n"] + 24.0 * case["targets"], "flops": 20.0 * case["n"] * case["targets"]}
-    n = case["systems"] * (case["n_lo"] + case["n_hi"]) / 2 if case["kind"] == "batch" else case["n"]
+    n = float(_sizes(case).sum()) if case["kind"] == "batch" else case["n"]
     limit = math.floor(math.sqrt(8) * case["s"])
     if case["model"] == "cube":
         depth = max(0, math.ceil(math.log(n / limit, 8))) if n > limit else 0
@@ -295,7 +296,7 @@ def _rk4(x, v, m, eps, dt, steps):
 
 def exact(case, seed):
     if case["kind"] == "batch":
-        sizes = _sizes(case, seed)
+        sizes = _sizes(case)
         if 4.0 * case["steps"] * float((sizes.astype(np.float64) ** 2).sum()) > EXACT_PAIRS:
             return None
         _, x, v = _batch_particles(case, seed)
