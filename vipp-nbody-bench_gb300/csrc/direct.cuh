@@ -13,6 +13,8 @@
 
 #include <cuda_runtime.h>
 
+#include "rinv.cuh"
+
 namespace gb {
 
 struct SoA {
@@ -36,7 +38,7 @@ constexpr int kDirectTB = 256;
 // an index outside [0, n) is not dereferenced and its result is NaN.
 template <class Pos, bool kCheckTargets = false>
 __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, const long long *__restrict__ targets,
-                                                           unsigned nt, unsigned nsplit, double Gm, double eps2,
+                                                           unsigned nt, unsigned nsplit, double Gm, double eps2, SoftInt soft,
                                                            double *__restrict__ part) {
     __shared__ double sx[kDirectTB], sy[kDirectTB], sz[kDirectTB];
     const unsigned k = blockIdx.x * kDirectTB + threadIdx.x;
@@ -66,9 +68,11 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
         for (unsigned q = 0; q < cnt; ++q) {
             if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
             const double dx = sx[q] - tx, dy = sy[q] - ty, dz = sz[q] - tz;
-            const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-            const double ri = rsqrt(r2);
-            const double f = Gm * ri * ri * ri;
+            double f;
+            if (!rinv3(dx, dy, dz, soft, f)) {
+                const double ri = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
+                f = ri * ri * ri;
+            }
             ax += f * dx;
             ay += f * dy;
             az += f * dz;
@@ -78,9 +82,9 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
     if (act || bad) {
         if (bad) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
         double *o = part + static_cast<size_t>(blockIdx.y) * 3 * nt;
-        o[k] = ax;
-        o[nt + k] = ay;
-        o[2 * static_cast<size_t>(nt) + k] = az;
+        o[k] = Gm * ax;
+        o[nt + k] = Gm * ay;
+        o[2 * static_cast<size_t>(nt) + k] = Gm * az;
     }
 }
 

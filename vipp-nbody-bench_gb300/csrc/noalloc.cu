@@ -114,7 +114,8 @@ extern "C" int gb_direct_accel_noalloc(const double *x_dev, size_t n, const int6
     // so nothing left there by an earlier call needs clearing
     k_direct_part<AoS, true><<<grid, kDirectTB, 0, st>>>(AoS{x_dev}, static_cast<unsigned>(n),
                                                          reinterpret_cast<const long long *>(targets_dev),
-                                                         static_cast<unsigned>(nt), nsplit, G * m, eps * eps, slot.scratch);
+                                                         static_cast<unsigned>(nt), nsplit, G * m, eps * eps,
+                                                         soft_int(eps * eps), slot.scratch);
     k_direct_reduce<<<static_cast<unsigned>((nt + 255) / 256), 256, 0, st>>>(slot.scratch, static_cast<unsigned>(nt), nsplit,
                                                                              nullptr, a_dev);
     if (cudaGetLastError() != cudaSuccess) return GB_ERR_CUDA;

@@ -20,6 +20,7 @@
 // and the reference's G, fmm.hpp:539, multiply the sum once); per-batch FP32
 // partial sums folded into a compensated (Kahan) per-target accumulator.
 #include "direct.cuh"
+#include "rinv.cuh"
 #include "workspace.cuh"
 
 #ifndef GB_P2P_CARVEOUT_MAX
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
                                                             unsigned *queue, const unsigned *__restrict__ rng_off,
                                                             const unsigned *__restrict__ rng_len, const uint2 *__restrict__ ranges,
                                                             const double *__restrict__ xs, const unsigned *__restrict__ src_total,
-                                                            double *__restrict__ part, double Gm, double eps2,
+                                                            double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ nearv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
     __shared__ double red[kP2PWarps][3][32];
@@ -289,10 +290,13 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
             if (tact)
                 for (unsigned k = grp; k < cnt; k += g) {
                     const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
-                    const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                    double ri = rsqrt(r2);
-                    if (!kSoft) ri = r2 > 0.0 ? ri : 0.0;
-                    const double f = ri * ri * ri;
+                    double f;
+                    if (!rinv3(dx, dy, dz, soft, f)) {
+                        const double r2 = dx * dx + dy * dy + dz * dz + eps2;
+                        double ri = rsqrt(r2);
+                        if (!kSoft) ri = r2 > 0.0 ? ri : 0.0;
+                        f = ri * ri * ri;
+                    }
                     ax += f * dx;
                     ay += f * dy;
                     az += f * dz;
@@ -347,7 +351,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
                                                             unsigned *queue, const unsigned *__restrict__ rng_off,
                                                             const unsigned *__restrict__ rng_len, const uint2 *__restrict__ ranges,
                                                             const double *__restrict__ xs, const unsigned *__restrict__ src_total,
-                                                            double *__restrict__ part, double Gm, double eps2,
+                                                            double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ phiv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
     __shared__ double red[kP2PWarps][32];
@@ -382,7 +386,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
                 for (unsigned k = grp; k < cnt; k += g) {
                     if (jb + k == i) continue;
                     const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
-                    pot += 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+                    double f;
+                    if (!rinv1(dx, dy, dz, soft, f)) f = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+                    pot += f;
                 }
             __syncwarp();
             cur.advance();
@@ -435,7 +441,8 @@ void near_potential(Workspace &ws, double *phiv) {
     const unsigned gs = static_cast<unsigned>(ws.num_sms) * 8;
     const double Gm = ws.forest() ? 1.0 : ws.G * ws.m;
     k_p2p_phi<<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len, ws.ranges, ws.xs,
-                                                ws.src_total, static_cast<double *>(ws.part), Gm, ws.eps * ws.eps, phiv, ws.n);
+                                                ws.src_total, static_cast<double *>(ws.part), Gm, ws.eps * ws.eps,
+                                                soft_int(ws.eps * ws.eps), phiv, ws.n);
     k_p2p_phi_combine<<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, static_cast<const double *>(ws.part), Gm, phiv);
     ws.launches += 2;
     if (ws.forest()) {
@@ -505,12 +512,13 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
         const double Gm = ws.forest() ? 1.0 : ws.G * ws.m, eps2 = ws.eps * ws.eps;
         auto *o = static_cast<double *>(ws.nearf);
         auto *pd = static_cast<double *>(ws.part);
+        const SoftInt si = soft_int(eps2);
         if (soft)
             k_p2p_f64<true><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len,
-                                                              ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, o, ws.n);
+                                                              ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, si, o, ws.n);
         else
             k_p2p_f64<false><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len,
-                                                               ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, o, ws.n);
+                                                               ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, si, o, ws.n);
     }
     ws.launches += 1;
     timer_end(ws, kTP2P);
@@ -540,7 +548,7 @@ void direct_sum(Workspace &ws, const double *x_orig, const long long *targets, u
                 double *part, unsigned nsplit) {
     const dim3 grid((nt + kDirectTB - 1) / kDirectTB, nsplit);
     k_direct_part<SoA><<<grid, kDirectTB, 0, ws.st>>>(SoA{x_orig, ws.n}, ws.n, targets, nt, nsplit, ws.G * ws.m,
-                                                     ws.eps * ws.eps, part);
+                                                     ws.eps * ws.eps, soft_int(ws.eps * ws.eps), part);
     k_direct_reduce<<<(nt + 255) / 256, 256, 0, ws.st>>>(part, nt, nsplit, out_soa, nullptr);
     ws.launches += 2;
 }
