@@ -282,6 +282,17 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
         ws.soft_corr = c;
         ws.soft_corr_cap = ws.n_cap;
     }
+    if (!ws.mixed) {
+        // class-group sums of the FP64 M2L's tiles while the tree is small
+        const unsigned tiles = std::min(gb::kM2LSplitTiles, gb::m2l_f64_tiles(ws));
+        if (tiles > ws.m2l_part_tiles || ws.p > ws.m2l_part_p) {
+            ++ctx->epoch;
+            GB_TRY(dalloc(ws.m2l_part, gb::m2l_f64_part_doubles(ws.p) * tiles));
+            GB_TRY(dalloc(ws.m2l_pcnt, tiles));
+            GB_TRY(cudaMemsetAsync(ws.m2l_pcnt, 0, sizeof(unsigned) * tiles, ws.st));
+            ws.m2l_part_tiles = tiles, ws.m2l_part_p = ws.p;
+        }
+    }
     if (ws.m2l_tensor) {
         // split expansions of the tensor-core M2L and their TMA map
         const int kp = gb::m2l_tc_row_floats(ws.p);
@@ -443,7 +454,7 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
         cudaEventRecord(ws.ev_join3, ws.st3);
     }
     gb::build_operators(ws);
-    if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : gb::kM2LTileCC);
+    if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : ws.mixed ? gb::kM2LTileCC : gb::kM2LTileF64);
     gb::upward_pass(ws);
     if (ws.m2l_tensor)
         gb::m2l_pass_tc(ws);
@@ -731,7 +742,7 @@ void gb_destroy(gb_ctx *ctx) {
                     ws.split_cell, ws.c_begin, ws.c_end, ws.c_parent, ws.c_child, ws.c_level, ws.c_path, ws.c_coord,
                     ws.c_box, ws.c_ctr, ws.Mexp, ws.Lexp, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                     ws.flag, ws.flag_off, ws.leaves, ws.rng_cnt, ws.rng_off, ws.rng_len, ws.ranges, ws.chunk_cnt,
-                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
+                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.m2l_part, ws.m2l_pcnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
                     ctx->d_direct, ws.seg, ws.psys, ws.c_sys, ws.sys_par, ws.mkeys, ws.etile, ws.oct_list, ws.otile,
                     ws.ocnt, ws.soft_corr};
     for (void *b : bufs) dfree(b);

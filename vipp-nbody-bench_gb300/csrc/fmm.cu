@@ -1000,7 +1000,9 @@ void dispatch_p(Workspace &ws, int which, double *farphi = nullptr) {
     case PP:                             \
         if (which == 5) launch_l2p_phi<PP, T>(ws, farphi); \
         if (which == 0) launch_p2m<PP, T>(ws); \
-        if (which == 1) launch_m2l<PP, T>(ws); \
+        if constexpr (sizeof(T) == 4) {  \
+            if (which == 1) launch_m2l<PP, T>(ws); \
+        }                                \
         if (which == 2) launch_l2p<PP, T>(ws); \
         if (which == 3) launch_m2m_levels<PP, T>(ws); \
         if (which == 4) launch_l2l_levels<PP, T>(ws); \
@@ -1074,7 +1076,7 @@ void m2l_pass(Workspace &ws) {
     if (ws.mixed)
         dispatch_p<float>(ws, 1);
     else
-        dispatch_p<double>(ws, 1);
+        m2l_pass_f64(ws);
     timer_end(ws, kTM2L);
 }
 

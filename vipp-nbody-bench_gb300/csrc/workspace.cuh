@@ -152,6 +152,11 @@ struct Workspace {
     bool ms_bf16 = false;     // the split form tmap_ms was encoded for
     CUtensorMap tmap_ms{};    // TMA map of ms_tc
 
+    double *m2l_part = nullptr;   // FP64 M2L: class-group sums of small trees' tiles (m2l_fp64.cu)
+    unsigned *m2l_pcnt = nullptr; // [m2l_part_tiles] finished groups of a tile, zero between evaluations
+    unsigned m2l_part_tiles = 0;  // tiles the two are sized for
+    int m2l_part_p = 0;           // and the expansion order
+
     // device-side info and device-resident counters
     TreeInfo *info = nullptr;
     unsigned *d_counts = nullptr;  // [kNumCounts]: 0 n, 1 S, 2 C, 3 leaves, 4 ranges, 5 items,
@@ -182,7 +187,11 @@ inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 inline const int *forest_cells(const Workspace &ws) { return ws.forest() ? ws.c_sys : nullptr; }
 constexpr int kM2LTileTC = 128;  // target octets per tensor-core M2L tile (m2l_tc.cu)
 constexpr int kZeroRows = 32;    // zero rows after the split expansions (one per row quad of a tile)
-constexpr int kM2LTileCC = 64;   // per CUDA-core M2L tile (fmm.cu)
+constexpr int kM2LTileCC = 64;   // per FP32 CUDA-core M2L tile (fmm.cu)
+constexpr int kM2LTileF64 = 32;  // per FP64 M2L tile (m2l_fp64.cu)
+// FP64 M2L tiles (32 targets of one octant) up to which a tile's class groups
+// run as blocks of their own: two blocks on each of the 152 SMs
+constexpr unsigned kM2LSplitTiles = 304;
 constexpr int kOpM2M = 343;  // op index of M2M octant 0
 constexpr int kOpL2L = 351;  // op index of L2L octant 0
 constexpr int kNumOps = 359;
@@ -195,7 +204,10 @@ size_t m2l_table_bytes(int p);
 inline size_t zf_table_floats(int p) { return static_cast<size_t>(kNumOps) * (2 * p + 1) * (2 * p + 1); }  // per system
 void build_m2l_table(Workspace &ws);          // fill m2l_tab for ws.p (once per p, outside step graphs)
 void upward_pass(Workspace &ws);              // P2M + M2M
-void m2l_pass(Workspace &ws);                 // M2L into L (CUDA cores)
+void m2l_pass(Workspace &ws);                 // M2L into L (CUDA cores, FP32)
+void m2l_pass_f64(Workspace &ws);             // M2L into L (FP64)
+unsigned m2l_f64_tiles(const Workspace &ws);  // bound of the tiles of ws.c_cap cells
+size_t m2l_f64_part_doubles(int p);           // class-group sums of one tile
 void m2l_pass_tc(Workspace &ws);              // M2L into L (tensor cores, mixed)
 bool m2l_tc_supported(int p);
 size_t m2l_tc_image_floats(int p);
