@@ -703,6 +703,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, GB_FAR_MIN_BLOC
     // tile reaches no cluster barrier and skips loading its operator
     if (static_cast<int>(blockIdx.x) / 8 >= tiles) return;
     tile_clear<P, T>(A);
+    __syncthreads();  // Op is cleared before any thread loads its part of the operator
     int loaded = -1;  // system whose operator is in Op
     const int nclusters = static_cast<int>(gridDim.x) / 8;
     for (int w = static_cast<int>(blockIdx.x) / 8; w < tiles; w += nclusters) {  // same w in all 8 CTAs
