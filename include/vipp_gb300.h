@@ -287,14 +287,14 @@ GB_API int gb_direct_accel_noalloc(const double *x_dev, size_t n, const int64_t 
 typedef struct gb_tuning {
     int p2p_blocks;      /* P2P blocks per SM when the near field runs alone, 1..16 (default 8) */
     int p2p_blocks_conc; /* P2P blocks per SM launched beside the far field, 0..16 (default 8) */
-    int p2p_slice;       /* near-field sources per P2P work item, 1024..65536 (default 8192) */
+    int p2p_slice;       /* near-field sources per P2P work item, 1024..65536 (default 8192);
+                            small systems take shorter ones (n / 8, FP64 n / 32) */
     int m2l_ctas_pct;    /* tensor-core M2L CTAs, percent of the SMs, 10..100 (default 100) */
     int serial;          /* 1: the near field after the far field on one stream (default 0) */
     int leaf_s;          /* GB_MODE_ACCURATE: leaf parameter used instead of the config's s
                             (0: the config's s) */
-    int p2p_occupancy;   /* mixed P2P kernel build: 8 (registers budgeted for 8 blocks
-                            per SM, default; 0 means 8) or 6 (80 registers, more work
-                            in flight per warp); same results either way */
+    int p2p_occupancy;   /* 8 (default; 0 means 8) or 6: named two builds of the mixed P2P
+                            kernel; one build (80 registers) now serves both */
 } gb_tuning;
 GB_API int gb_set_tuning(gb_ctx *ctx, const gb_tuning *t);
 GB_API int gb_get_tuning(const gb_ctx *ctx, gb_tuning *out);

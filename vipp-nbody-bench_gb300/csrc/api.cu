@@ -118,7 +118,6 @@ void apply_config(gb_ctx *ctx) {
     ws.serial = (ctx->cfg.flags & GB_FLAG_SERIAL) != 0 || ctx->tune.serial != 0;
     ws.p2p_blocks = static_cast<unsigned>(ctx->tune.p2p_blocks);
     ws.p2p_blocks_conc = static_cast<unsigned>(ctx->tune.p2p_blocks_conc);
-    ws.p2p_occ = ctx->tune.p2p_occupancy == 6 ? 6 : 8;
     ws.p2p_slice = static_cast<unsigned>(ctx->tune.p2p_slice);
     ws.m2l_ctas_pct = ctx->tune.m2l_ctas_pct;
     ws.accurate = ctx->cfg.mode == GB_MODE_ACCURATE;
@@ -141,7 +140,7 @@ int ensure_chunks(gb_ctx *ctx, unsigned need_items = 0, unsigned need_part = 0) 
         GB_TRY(dalloc(ws.chunks, ch));
         ws.ch_cap = ch;
     }
-    unsigned pc = ws.part_cap ? ws.part_cap : 4096u;
+    unsigned pc = ws.part_cap ? ws.part_cap : 16384u;
     if (need_part > pc) pc = need_part + need_part / 4;
     if (pc > ws.part_cap || !ws.part) {
         ++ctx->epoch;
@@ -237,7 +236,7 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
         GB_TRY(dalloc(ws.leaves, c));
         GB_TRY(dalloc(ws.rng_cnt, c + 1));
         GB_TRY(dalloc(ws.rng_off, c + 1));
-        GB_TRY(dalloc(ws.rng_len, c));
+        GB_TRY(dalloc(ws.leaf_rec, c));
         GB_TRY(dalloc(ws.chunk_cnt, c + 1));
         GB_TRY(dalloc(ws.chunk_off, c + 1));
         GB_TRY(dalloc(ws.src_total, c + 1));
@@ -741,7 +740,7 @@ void gb_destroy(gb_ctx *ctx) {
                     ws.perm0, ws.perm1, ws.inv, ws.xs, ws.ph, ws.pl, ws.nearf, ws.farf, ws.phis, ws.cnt, ws.off, ws.ent0, ws.ent1,
                     ws.split_cell, ws.c_begin, ws.c_end, ws.c_parent, ws.c_child, ws.c_level, ws.c_path, ws.c_coord,
                     ws.c_box, ws.c_ctr, ws.Mexp, ws.Lexp, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
-                    ws.flag, ws.flag_off, ws.leaves, ws.rng_cnt, ws.rng_off, ws.rng_len, ws.ranges, ws.chunk_cnt,
+                    ws.flag, ws.flag_off, ws.leaves, ws.rng_cnt, ws.rng_off, ws.leaf_rec, ws.ranges, ws.chunk_cnt,
                     ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.m2l_part, ws.m2l_pcnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
                     ctx->d_direct, ws.seg, ws.psys, ws.c_sys, ws.sys_par, ws.mkeys, ws.etile, ws.oct_list, ws.otile,
                     ws.ocnt, ws.soft_corr};

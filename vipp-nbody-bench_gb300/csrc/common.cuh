@@ -116,6 +116,21 @@ GB_HD void chunk_at(int n, int q, int &off, int &len) {
 // are added in slice order afterwards. This bounds the longest work item.
 constexpr int kSliceSources = 8192;  // default; the tuning may pick another length
 constexpr int kMaxSlices = 4095;
+// Small systems take shorter slices: their few leaves would leave most warps of
+// the GPU without an item (16,384 particles: about 900 items of 3,700 sources for
+// 3,648 resident warps). FP64 pairs hold the FP64 pipe for 384 cycles each, so
+// those slices are n / 32 sources, at least 128 (16,384 particles: near field
+// 3.68 -> 0.88 ms per evaluation, 4.65 without slices below 8,192); FP32 slices
+// are n / 8, at least 512 (3,001 particles 0.12 -> 0.025 ms), since shorter ones
+// cost a batch of many systems, whose items fill the GPU anyway, more than they
+// give (512 systems: 88.2 ms without, 91.4 with n / 32). The length follows from
+// the system's own particle count, so a forest's system sums its sources in the
+// same order as in a context of its own.
+GB_HD unsigned slice_length(unsigned n, unsigned slice, bool fp32) {
+    const unsigned lo = fp32 ? 512u : 128u, s = (fp32 ? n / 8 : n / 32) / 32 * 32;
+    const unsigned q = s < lo ? lo : s;
+    return q < slice ? q : slice;
+}
 GB_HD int slice_count(unsigned long long srcs, unsigned slice = kSliceSources) {
     const unsigned long long s = (srcs + slice - 1) / slice;
     return s < 1 ? 1 : (s > kMaxSlices ? kMaxSlices : static_cast<int>(s));

@@ -9,7 +9,9 @@
 // A warp streams the leaf's near-field source ranges through shared memory
 // 32 sources at a time, prefetching the next batch into registers while it
 // works on the current one; lanes read the staged sources with broadcast
-// shared-memory loads.
+// shared-memory loads, two sources per step on paired FP32 instructions in
+// chunks of every size (a slice's last batch is filled up with sources that add
+// nothing).
 //
 // Mixed precision (FP32): positions are kept as hi + lo float pairs relative
 // to the root-box centre; targets and staged sources are re-expressed relative
@@ -39,48 +41,44 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return r;
 }
 
-// Source-batch cursor over a slice [v0, v0 + len) of the concatenation of a
-// leaf's source ranges; batches never cross a range end.
-struct Cursor {
-    const uint2 *rng;
-    unsigned nr, r, b, end, rem;
-    __device__ __forceinline__ void start(const uint2 *ranges, unsigned n, unsigned v0, unsigned len) {
-        rng = ranges, nr = n, r = 0, rem = len, b = 0, end = 0;
-        for (; r < nr; ++r) {
-            const uint2 g = rng[r];
-            if (v0 < g.y - g.x) {
-                b = g.x + v0, end = g.y;
-                break;
-            }
-            v0 -= g.y - g.x;
-        }
-        if (rem == 0) r = nr;
-    }
-    __device__ __forceinline__ bool valid() const { return r < nr; }
-    __device__ __forceinline__ unsigned count() const { return min(min(32u, end - b), rem); }
-    __device__ __forceinline__ void advance() {
-        const unsigned c = count();
-        rem -= c, b += c;
-        if (rem == 0) {
-            r = nr;
-        } else if (b >= end && ++r < nr) {
-            const uint2 g = rng[r];
-            b = g.x, end = g.y;
-        }
-    }
-};
-
-// The same walk in full batches: up to 32 sources taken across range
-// boundaries, lane l getting the l-th (a batch is cut only at the slice's end,
-// so every batch but the last is full and takes the paired path). The state
-// is uniform over the warp; the loop runs once per range the batch touches.
+// Source batches of a slice [v0, v0 + len) of the concatenation of a leaf's
+// source ranges: up to 32 sources taken across range boundaries, lane l getting
+// the l-th (a batch is cut only at the slice's end). The state is uniform over
+// the warp; the ranges are read 32 at a time, one per lane, and handed around by
+// shuffles, so that neither finding the slice's start nor crossing into the next
+// range waits for a chain of dependent loads (a range holds ~155 sources at 4M).
 struct BatchCursor {
     const uint2 *rng;
-    unsigned nr, r, b, end, rem;
-    __device__ __forceinline__ void start(const uint2 *ranges, unsigned n, unsigned v0, unsigned len) {
-        Cursor c;
-        c.start(ranges, n, v0, len);
-        rng = c.rng, nr = c.nr, r = c.r, b = c.b, end = c.end, rem = c.rem;
+    uint2 mine;  // range r0 + lane
+    unsigned nr, r0, r, b, end, rem;
+    __device__ __forceinline__ void window(unsigned lane) {
+        mine = r0 + lane < nr ? rng[r0 + lane] : make_uint2(0, 0);
+    }
+    __device__ __forceinline__ void start(const uint2 *ranges, unsigned n, unsigned v0, unsigned len, unsigned lane) {
+        rng = ranges, nr = n, r0 = 0, rem = len, b = 0, end = 0;
+        window(lane);
+        while (true) {
+            unsigned cum = mine.y - mine.x;  // sources of this window's ranges up to and with this lane's
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, cum, o);
+                if (lane >= o) cum += y;
+            }
+            const unsigned past = __ballot_sync(0xffffffffu, cum > v0);
+            if (past) {
+                const int q = __ffs(past) - 1;
+                const unsigned at = __shfl_sync(0xffffffffu, mine.y - (cum - v0), q);
+                r = r0 + q, b = at, end = __shfl_sync(0xffffffffu, mine.y, q);
+                return;
+            }
+            v0 -= __shfl_sync(0xffffffffu, cum, 31);
+            r0 += 32;
+            if (r0 >= nr) {  // an empty slice
+                r = nr, rem = 0;
+                return;
+            }
+            window(lane);
+        }
     }
     // the next batch: its size, and this lane's source index (lane < size)
     __device__ __forceinline__ unsigned next(unsigned lane, unsigned &idx) {
@@ -91,8 +89,8 @@ struct BatchCursor {
             if (lane >= filled && lane < filled + take) idx = b + (lane - filled);
             filled += take, rem -= take, b += take;
             if (b >= end && ++r < nr) {
-                const uint2 g = rng[r];
-                b = g.x, end = g.y;
+                if (r - r0 == 32) r0 = r, window(lane);
+                b = __shfl_sync(0xffffffffu, mine.x, r - r0), end = __shfl_sync(0xffffffffu, mine.y, r - r0);
             }
         }
         return filled;
@@ -104,132 +102,131 @@ struct BatchCursor {
 struct Item {
     int li, t0, nt, sl, ns, pslot;
     unsigned v0, len;
-    __device__ __forceinline__ Item(const int4 w, const unsigned *src_total) {
-        li = w.x, t0 = w.y, nt = item_nt(w.z), sl = item_slice(w.z), ns = item_nslices(w.z), pslot = w.w;
-        const unsigned S = src_total[li];
+    __device__ __forceinline__ explicit Item(const int4 w)
+        : li(w.x), t0(w.y), nt(item_nt(w.z)), sl(item_slice(w.z)), ns(item_nslices(w.z)), pslot(w.w) {}
+    __device__ __forceinline__ void slice(unsigned S) {
         const unsigned per = (S + ns - 1) / ns;
         v0 = min(S, sl * per);
         len = min(per, S - v0);
     }
 };
 
+// A source pair (j, j') against a target on paired FP32 instructions (.f32x2);
+// each component rounds exactly like the scalar operation.
 template <bool kNewton, bool kSoft>
-__device__ __forceinline__ void pair_f32(const float4 s, float tx, float ty, float tz, float eps2, float &bx, float &by,
-                                         float &bz) {
-    const float dx = s.x - tx, dy = s.y - ty, dz = s.z - tz;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    float ri = rsqrt_ftz(r2);
-    if (kNewton) ri = ri * fmaf(-0.5f * r2 * ri, ri, 1.5f);
-    if (!kSoft) ri = r2 > 0.f ? ri : 0.f;
-    const float f = ri * (ri * ri);
-    bx = fmaf(dx, f, bx);
-    by = fmaf(dy, f, by);
-    bz = fmaf(dz, f, bz);
+__device__ __forceinline__ void pair2_f32(float2 x, float2 y, float2 z, float2 ntx, float2 nty, float2 ntz, float2 e2,
+                                          float2 &ax, float2 &ay, float2 &az) {
+    const float2 dx = __fadd2_rn(x, ntx), dy = __fadd2_rn(y, nty), dz = __fadd2_rn(z, ntz);
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+    float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+    if (kNewton) {
+        ri.x = ri.x * fmaf(-0.5f * r2.x * ri.x, ri.x, 1.5f);
+        ri.y = ri.y * fmaf(-0.5f * r2.y * ri.y, ri.y, 1.5f);
+    }
+    if (!kSoft) ri.x = r2.x > 0.f ? ri.x : 0.f, ri.y = r2.y > 0.f ? ri.y : 0.f;
+    const float2 f = __fmul2_rn(ri, __fmul2_rn(ri, ri));
+    ax = __ffma2_rn(dx, f, ax);
+    ay = __ffma2_rn(dy, f, ay);
+    az = __ffma2_rn(dz, f, az);
 }
 
-// Register budgets of the mixed-precision kernel (tuning knob p2p_occupancy):
-// compiled for 8 resident blocks per SM (64 registers) or for 6 (80
-// registers: more pair terms in flight per warp, which pays while P2P shares
-// the SMs with the far field on 2 blocks per SM). Both fit beside the far
-// field's kernels (a 96-register build kept the cluster M2M from starting
-// beside P2P and serialised the two). The same arithmetic either way, so
-// the same results bit for bit.
-template <bool kNewton, bool kSoft, int kMinBlocks>
-__global__ void __launch_bounds__(kP2PWarps * 32, kMinBlocks) k_p2p_f32(const int4 *__restrict__ chunks, const unsigned *counts,
-                                                            unsigned *queue, const int *__restrict__ leaves,
-                                                            const double *__restrict__ c_ctr,
-                                                            const TreeInfo *__restrict__ info, const int *__restrict__ c_sys,
-                                                            const unsigned *__restrict__ rng_off,
-                                                            const unsigned *__restrict__ rng_len, const uint2 *__restrict__ ranges,
-                                                            const float4 *__restrict__ ph, const float4 *__restrict__ pl,
-                                                            const unsigned *__restrict__ src_total, float *__restrict__ part,
-                                                            float Gm, float eps2, float *__restrict__ nearv, unsigned n) {
-    __shared__ float4 src[kP2PWarps][32];
-    __shared__ float4 srcxy[kP2PWarps][16];  // sources 2m, 2m+1 as {x, x', y, y'}
-    __shared__ float2 srcz[kP2PWarps][16];   // and {z, z'}
+// Coordinate of the sources that fill up a slice's last batch: r^-3 of 1e18
+// underflows to 0, so they add exactly nothing.
+constexpr float kNowhere = 1e18f;
+
+// Compiled for 6 resident blocks per SM (80 registers). Bound by the FMA pipe
+// and what a batch costs beside its pairs: the pair loop alone reaches 8.9 pairs
+// per clock and SM (11 FP32 operations a pair: 84% of the measured FMA rate), with
+// the staging of a batch and the compensated sums 8.0, with the 94% of lanes that
+// a leaf's chunks fill 7.5; the kernel runs at 7.0 (4M Plummer, 1.03e10 pairs: 4.83
+// ms, 4.92 before; 1M unit cube 0.475 -> 0.465; 1M at p = 10 2.06 -> 1.96). A
+// 64-register build (8 blocks) spills 24 bytes and measured 1-5% slower on every
+// workload; a 96-register build kept the cluster M2M from starting beside P2P.
+template <bool kNewton, bool kSoft>
+__global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__restrict__ chunks, const unsigned *counts,
+                                                            unsigned *queue, const LeafRec *__restrict__ recs,
+                                                            const uint2 *__restrict__ ranges, const float4 *__restrict__ ph,
+                                                            const float4 *__restrict__ pl, float *__restrict__ part, float Gm,
+                                                            float eps2, float *__restrict__ nearv, unsigned n) {
+    __shared__ __align__(16) float src[kP2PWarps][3][32];  // the staged batch, leaf-relative
     __shared__ float red[kP2PWarps][3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
-    float *pxy = reinterpret_cast<float *>(srcxy[w]);
-    float *pz = reinterpret_cast<float *>(srcz[w]);
+    unsigned ci = 0;
+    if (lane == 0) ci = atomicAdd(queue, 1u);
     while (true) {
-        unsigned ci = 0;
-        if (lane == 0) ci = atomicAdd(queue, 1u);
         ci = __shfl_sync(0xffffffffu, ci, 0);
         if (ci >= nch) break;
-        const Item it(chunks[ci], src_total);
+        Item it(chunks[ci]);
+        const LeafRec rec = recs[it.li];
+        it.slice(rec.src_total);
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
         const int t = lane - grp * nt;
         const bool tact = grp < g;
         const int i = it.t0 + t;
-        const int leaf = leaves[it.li];
-        const RootC cc = leaf_centre(c_ctr, leaf, info + cell_system(c_sys, leaf));
-        float tx = 0, ty = 0, tz = 0;
+        // minus the leaf centre: a position is (hi - centre hi) + (lo - centre lo)
+        const float2 chxy = make_float2(-rec.hx, -rec.hy), clxy = make_float2(-rec.lx, -rec.ly);
+        const float chz = -rec.hz, clz = -rec.lz;
+        float2 txy = make_float2(0.f, 0.f);
+        float tz = 0;
         if (tact) {
             const float4 h = ph[i], l = pl[i];
-            tx = (h.x - cc.hx) + (l.x - cc.lx);
-            ty = (h.y - cc.hy) + (l.y - cc.ly);
-            tz = (h.z - cc.hz) + (l.z - cc.lz);
+            txy = __fadd2_rn(__fadd2_rn(make_float2(h.x, h.y), chxy), __fadd2_rn(make_float2(l.x, l.y), clxy));
+            tz = (h.z + chz) + (l.z + clz);
         }
         float sx = 0, sy = 0, sz = 0, kx = 0, ky = 0, kz = 0;  // Kahan sums and compensations
         BatchCursor cur;
-        cur.start(ranges + rng_off[it.li], rng_len[it.li], it.v0, it.len);
+        cur.start(ranges + rec.rng_off, rec.rng_len, it.v0, it.len, static_cast<unsigned>(lane));
         float4 h = make_float4(0, 0, 0, 0), l = h;
         unsigned sidx;
         unsigned cnt = cur.next(static_cast<unsigned>(lane), sidx);
         if (static_cast<unsigned>(lane) < cnt) h = ph[sidx], l = pl[sidx];
-        const float2 ntx = make_float2(-tx, -tx), nty = make_float2(-ty, -ty), ntz = make_float2(-tz, -tz);
+        const float2 ntx = make_float2(-txy.x, -txy.x), nty = make_float2(-txy.y, -txy.y), ntz = make_float2(-tz, -tz);
         const float2 e2 = make_float2(eps2, eps2);
+        bool taken = false;
         while (cnt) {
-            if (static_cast<unsigned>(lane) < cnt) {
-                const float qx = (h.x - cc.hx) + (l.x - cc.lx), qy = (h.y - cc.hy) + (l.y - cc.ly),
-                            qz = (h.z - cc.hz) + (l.z - cc.lz);
-                src[w][lane] = make_float4(qx, qy, qz, 0.f);
-                pxy[(lane >> 1) * 4 + (lane & 1)] = qx;
-                pxy[(lane >> 1) * 4 + 2 + (lane & 1)] = qy;
-                pz[(lane >> 1) * 2 + (lane & 1)] = qz;
-            }
+            const bool on = static_cast<unsigned>(lane) < cnt;
+            const float2 xy = __fadd2_rn(__fadd2_rn(make_float2(h.x, h.y), chxy), __fadd2_rn(make_float2(l.x, l.y), clxy));
+            src[w][0][lane] = on ? xy.x : kNowhere;
+            src[w][1][lane] = xy.y;
+            src[w][2][lane] = (h.z + chz) + (l.z + clz);
             __syncwarp();
-            const unsigned now = cnt;
             cnt = cur.next(static_cast<unsigned>(lane), sidx);  // prefetch the next batch while this one is computed
             if (static_cast<unsigned>(lane) < cnt) h = ph[sidx], l = pl[sidx];
-            float bx = 0, by = 0, bz = 0;
-            if (g == 1 && now == 32) {
-                // two sources per step on paired FP32 instructions (.f32x2);
-                // each component rounds exactly like the scalar operation
-                float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+            if (cur.rem == 0 && !taken) {  // the slice's last batch is on its way: take the next item
+                taken = true;
+                if (lane == 0) ci = atomicAdd(queue, 1u);
+            }
+            float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+            if (g == 1) {
 #pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                    const float4 q = srcxy[w][m];
-                    const float2 dx = __fadd2_rn(make_float2(q.x, q.y), ntx);
-                    const float2 dy = __fadd2_rn(make_float2(q.z, q.w), nty);
-                    const float2 dz = __fadd2_rn(srcz[w][m], ntz);
-                    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-                    float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-                    if (kNewton) {
-                        ri.x = ri.x * fmaf(-0.5f * r2.x * ri.x, ri.x, 1.5f);
-                        ri.y = ri.y * fmaf(-0.5f * r2.y * ri.y, ri.y, 1.5f);
-                    }
-                    if (!kSoft) ri.x = r2.x > 0.f ? ri.x : 0.f, ri.y = r2.y > 0.f ? ri.y : 0.f;
-                    const float2 f = __fmul2_rn(ri, __fmul2_rn(ri, ri));
-                    ax = __ffma2_rn(dx, f, ax);
-                    ay = __ffma2_rn(dy, f, ay);
-                    az = __ffma2_rn(dz, f, az);
+                for (int m = 0; m < 8; ++m) {
+                    const float4 x = reinterpret_cast<const float4 *>(src[w][0])[m];
+                    const float4 y = reinterpret_cast<const float4 *>(src[w][1])[m];
+                    const float4 z = reinterpret_cast<const float4 *>(src[w][2])[m];
+                    pair2_f32<kNewton, kSoft>(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), ntx, nty, ntz,
+                                              e2, ax, ay, az);
+                    pair2_f32<kNewton, kSoft>(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), ntx, nty, ntz,
+                                              e2, ax, ay, az);
                 }
-                bx = ax.x + ax.y, by = ay.x + ay.y, bz = az.x + az.y;
-            } else if (tact) {
-                for (unsigned k = grp; k < now; k += g) pair_f32<kNewton, kSoft>(src[w][k], tx, ty, tz, eps2, bx, by, bz);
+            } else {
+#pragma unroll 2
+                for (int m = tact ? grp : 16; m < 16; m += g)
+                    pair2_f32<kNewton, kSoft>(reinterpret_cast<const float2 *>(src[w][0])[m],
+                                              reinterpret_cast<const float2 *>(src[w][1])[m],
+                                              reinterpret_cast<const float2 *>(src[w][2])[m], ntx, nty, ntz, e2, ax, ay, az);
             }
             __syncwarp();
-            float y = bx - kx, tt = sx + y;
+            float y = (ax.x + ax.y) - kx, tt = sx + y;
             kx = (tt - sx) - y, sx = tt;
-            y = by - ky, tt = sy + y;
+            y = (ay.x + ay.y) - ky, tt = sy + y;
             ky = (tt - sy) - y, sy = tt;
-            y = bz - kz, tt = sz + y;
+            y = (az.x + az.y) - kz, tt = sz + y;
             kz = (tt - sz) - y, sz = tt;
         }
+        if (!taken && lane == 0) ci = atomicAdd(queue, 1u);  // an empty slice
         sx -= kx, sy -= ky, sz -= kz;
         if (g > 1) {
             red[w][0][lane] = sx, red[w][1][lane] = sy, red[w][2][lane] = sz;
@@ -253,9 +250,8 @@ __global__ void __launch_bounds__(kP2PWarps * 32, kMinBlocks) k_p2p_f32(const in
 
 template <bool kSoft>
 __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restrict__ chunks, const unsigned *counts,
-                                                            unsigned *queue, const unsigned *__restrict__ rng_off,
-                                                            const unsigned *__restrict__ rng_len, const uint2 *__restrict__ ranges,
-                                                            const double *__restrict__ xs, const unsigned *__restrict__ src_total,
+                                                            unsigned *queue, const LeafRec *__restrict__ recs,
+                                                            const uint2 *__restrict__ ranges, const double *__restrict__ xs,
                                                             double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ nearv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
@@ -267,7 +263,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
         if (lane == 0) ci = atomicAdd(queue, 1u);
         ci = __shfl_sync(0xffffffffu, ci, 0);
         if (ci >= nch) break;
-        const Item it(chunks[ci], src_total);
+        Item it(chunks[ci]);
+        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total
+        it.slice(rec.z);
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
@@ -276,18 +274,18 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
         const int i = it.t0 + t;
         const double tx = tact ? xs[i] : 0.0, ty = tact ? xs[n + i] : 0.0, tz = tact ? xs[2 * static_cast<size_t>(n) + i] : 0.0;
         double ax = 0, ay = 0, az = 0;
-        Cursor cur;
-        cur.start(ranges + rng_off[it.li], rng_len[it.li], it.v0, it.len);
-        while (cur.valid()) {
-            const unsigned cnt = cur.count();
+        BatchCursor cur;
+        cur.start(ranges + rec.x, rec.y, it.v0, it.len, static_cast<unsigned>(lane));
+        unsigned j;
+        for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
             if (static_cast<unsigned>(lane) < cnt) {
-                const unsigned j = cur.b + lane;
                 src[w][0][lane] = xs[j];
                 src[w][1][lane] = xs[n + j];
                 src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
             }
             __syncwarp();
             if (tact)
+#pragma unroll 2
                 for (unsigned k = grp; k < cnt; k += g) {
                     const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
                     double f;
@@ -302,7 +300,6 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
                     az += f * dz;
                 }
             __syncwarp();
-            cur.advance();
         }
         if (g > 1) {
             red[w][0][lane] = ax, red[w][1][lane] = ay, red[w][2][lane] = az;
@@ -348,13 +345,13 @@ __global__ void k_p2p_combine(const int4 *__restrict__ chunks, const unsigned *c
 // indices) of (|x_j - x_i|^2 + eps^2)^(-1/2). Split items leave per-slice
 // partial sums in part[slot][0..31]; k_p2p_phi_combine adds them in slice order.
 __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restrict__ chunks, const unsigned *counts,
-                                                            unsigned *queue, const unsigned *__restrict__ rng_off,
-                                                            const unsigned *__restrict__ rng_len, const uint2 *__restrict__ ranges,
-                                                            const double *__restrict__ xs, const unsigned *__restrict__ src_total,
+                                                            unsigned *queue, const LeafRec *__restrict__ recs,
+                                                            const uint2 *__restrict__ ranges, const double *__restrict__ xs,
                                                             double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ phiv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
     __shared__ double red[kP2PWarps][32];
+    __shared__ unsigned sidx[kP2PWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
     while (true) {
@@ -362,7 +359,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
         if (lane == 0) ci = atomicAdd(queue, 1u);
         ci = __shfl_sync(0xffffffffu, ci, 0);
         if (ci >= nch) break;
-        const Item it(chunks[ci], src_total);
+        Item it(chunks[ci]);
+        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total
+        it.slice(rec.z);
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
@@ -371,27 +370,26 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
         const unsigned i = static_cast<unsigned>(it.t0 + t);
         const double tx = tact ? xs[i] : 0.0, ty = tact ? xs[n + i] : 0.0, tz = tact ? xs[2 * static_cast<size_t>(n) + i] : 0.0;
         double pot = 0;
-        Cursor cur;
-        cur.start(ranges + rng_off[it.li], rng_len[it.li], it.v0, it.len);
-        while (cur.valid()) {
-            const unsigned cnt = cur.count(), jb = cur.b;
+        BatchCursor cur;
+        cur.start(ranges + rec.x, rec.y, it.v0, it.len, static_cast<unsigned>(lane));
+        unsigned j;
+        for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
             if (static_cast<unsigned>(lane) < cnt) {
-                const unsigned j = jb + lane;
                 src[w][0][lane] = xs[j];
                 src[w][1][lane] = xs[n + j];
                 src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
+                sidx[w][lane] = j;
             }
             __syncwarp();
             if (tact)
                 for (unsigned k = grp; k < cnt; k += g) {
-                    if (jb + k == i) continue;
+                    if (sidx[w][k] == i) continue;
                     const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
                     double f;
                     if (!rinv1(dx, dy, dz, soft, f)) f = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
                     pot += f;
                 }
             __syncwarp();
-            cur.advance();
         }
         if (g > 1) {
             red[w][lane] = pot;
@@ -440,8 +438,8 @@ void near_potential(Workspace &ws, double *phiv) {
     cudaMemsetAsync(ws.queue, 0, sizeof(unsigned), ws.st);
     const unsigned gs = static_cast<unsigned>(ws.num_sms) * 8;
     const double Gm = ws.forest() ? 1.0 : ws.G * ws.m;
-    k_p2p_phi<<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len, ws.ranges, ws.xs,
-                                                ws.src_total, static_cast<double *>(ws.part), Gm, ws.eps * ws.eps,
+    k_p2p_phi<<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.xs,
+                                                static_cast<double *>(ws.part), Gm, ws.eps * ws.eps,
                                                 soft_int(ws.eps * ws.eps), phiv, ws.n);
     k_p2p_phi_combine<<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, static_cast<const double *>(ws.part), Gm, phiv);
     ws.launches += 2;
@@ -456,45 +454,31 @@ void near_potential(Workspace &ws, double *phiv) {
 // launches (on any streams) may drain the same queue, each item is taken once.
 // p2p_finish adds the slices of split items after all of them.
 
-template <int kMinBlocks>
 void p2p_f32_carveout() {
     // keep the SMs that run P2P configured for full shared memory, so far-field
     // kernels (the tensor-core M2L: up to 206 KB) can start beside the P2P blocks
-    cudaFuncSetAttribute(k_p2p_f32<false, true, kMinBlocks>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<false, false, kMinBlocks>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<true, true, kMinBlocks>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<true, false, kMinBlocks>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(k_p2p_f32<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(k_p2p_f32<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(k_p2p_f32<true, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(k_p2p_f32<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
 void p2p_pass(Workspace &ws, unsigned per_sm) {
     if (per_sm == 0) return;
     timer_begin(ws, kTP2P);
 #if GB_P2P_CARVEOUT_MAX
-    p2p_f32_carveout<8>();
-    p2p_f32_carveout<6>();
+    p2p_f32_carveout();
 #endif
-    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * per_sm, ceil_div(ws.n, 128));
+    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * per_sm, ceil_div(ws.ch_cap, kP2PWarps));
     const bool soft = ws.eps > 0;
     if (ws.mixed) {
         const float eps2 = static_cast<float>(ws.eps * ws.eps);
         const float Gm = ws.forest() ? 1.0f : static_cast<float>(ws.G * ws.m);  // a forest scales in p2p_finish
         auto *o = static_cast<float *>(ws.nearf);
         auto *pf = static_cast<float *>(ws.part);
-#define GB_P2P32_MB(NW, SF, MB)                                                                                  \
-    k_p2p_f32<NW, SF, MB><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaves, ws.c_ctr,    \
-                                                            ws.info, forest_cells(ws), ws.rng_off, ws.rng_len,        \
-                                                            ws.ranges, ws.ph, ws.pl, ws.src_total, pf, Gm, eps2, o, ws.n)
-#define GB_P2P32(NW, SF)             \
-    do {                             \
-        if (ws.p2p_occ == 6)         \
-            GB_P2P32_MB(NW, SF, 6);  \
-        else                         \
-            GB_P2P32_MB(NW, SF, 8);  \
-    } while (0)
+#define GB_P2P32(NW, SF)                                                                                             \
+    k_p2p_f32<NW, SF><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.ph, \
+                                                        ws.pl, pf, Gm, eps2, o, ws.n)
         if (ws.p2p_newton) {
             if (soft)
                 GB_P2P32(true, true);
@@ -507,25 +491,24 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
                 GB_P2P32(false, false);
         }
 #undef GB_P2P32
-#undef GB_P2P32_MB
     } else {
         const double Gm = ws.forest() ? 1.0 : ws.G * ws.m, eps2 = ws.eps * ws.eps;
         auto *o = static_cast<double *>(ws.nearf);
         auto *pd = static_cast<double *>(ws.part);
         const SoftInt si = soft_int(eps2);
         if (soft)
-            k_p2p_f64<true><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len,
-                                                              ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, si, o, ws.n);
+            k_p2p_f64<true><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges,
+                                                              ws.xs, pd, Gm, eps2, si, o, ws.n);
         else
-            k_p2p_f64<false><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.rng_off, ws.rng_len,
-                                                               ws.ranges, ws.xs, ws.src_total, pd, Gm, eps2, si, o, ws.n);
+            k_p2p_f64<false><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges,
+                                                               ws.xs, pd, Gm, eps2, si, o, ws.n);
     }
     ws.launches += 1;
     timer_end(ws, kTP2P);
 }
 
 void p2p_finish(Workspace &ws) {
-    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.n, 128));
+    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.ch_cap, 8));
     const bool forest = ws.forest();
     const double Gm = forest ? 1.0 : ws.G * ws.m;
     if (ws.mixed)

@@ -765,10 +765,16 @@ __global__ void k_lists(const uint64_t *__restrict__ ent, const unsigned *counts
 // ancestors from the root down, then its own (the inherited list of
 // solver_ref.hpp:126 followed by the cell's additions). Each entry is a
 // subtree, i.e. a contiguous particle range in tree order.
+__device__ __forceinline__ unsigned leaf_slice(int c, unsigned slice, bool fp32, unsigned n, const unsigned *seg,
+                                               const int *c_sys) {
+    return slice_length(seg ? seg[c_sys[c] + 1] - seg[c_sys[c]] : n, slice, fp32);
+}
+
 __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
                             const int *__restrict__ c_begin, const int *__restrict__ c_end,
                             const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt, unsigned *rng_cnt,
-                            unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice) {
+                            unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, bool fp32, unsigned n,
+                            const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
     const unsigned NL = counts[3];
     for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < NL; li += gridDim.x * blockDim.x) {
         const int c = leaves[li];
@@ -784,7 +790,7 @@ __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *coun
                 }
             }
         rng_cnt[li] = tot;
-        const unsigned ns = nt > 0 ? static_cast<unsigned>(slice_count(srcs, slice)) : 1u;
+        const unsigned ns = nt > 0 ? static_cast<unsigned>(slice_count(srcs, leaf_slice(c, slice, fp32, n, seg, c_sys))) : 1u;
         chunk_cnt[li] = static_cast<unsigned>(chunk_count(nt)) * ns;
         part_cnt[li] = ns > 1 ? static_cast<unsigned>(chunk_count(nt)) * ns : 0u;
         src_total[li] = static_cast<unsigned>(srcs < 0xffffffffull ? srcs : 0xffffffffull);
@@ -799,9 +805,11 @@ __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *coun
 __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
                            const int *__restrict__ c_parent, const int *__restrict__ c_begin, const int *__restrict__ c_end,
                            const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt,
-                           const unsigned *__restrict__ rng_off, unsigned *rng_len, uint2 *ranges,
+                           const unsigned *__restrict__ rng_off, LeafRec *leaf_rec, const double *__restrict__ c_ctr,
+                           uint2 *ranges,
                            const unsigned *__restrict__ chunk_off, int4 *chunks, const unsigned *__restrict__ src_total,
-                           const unsigned *__restrict__ part_off, unsigned part_cap, TreeInfo *info, unsigned slice) {
+                           const unsigned *__restrict__ part_off, unsigned part_cap, TreeInfo *info, unsigned slice, bool fp32, unsigned n,
+                           const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         counts[7] = counts[5];  // requested sizes, kept for the host when they overflow
         const bool over = counts[4] > r_cap || counts[5] > ch_cap || counts[8] > part_cap;
@@ -815,8 +823,7 @@ __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, uns
         const int c = leaves[li];
         const int b = c_begin[c], e = c_end[c];
         if (e == b) {
-            rng_len[li] = 0;
-            continue;
+            continue;  // no work item names it
         }
         int anc[kMaxLevel + 2];
         int na = 0;
@@ -855,10 +862,17 @@ __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, uns
                 overflow = true;
             ++k;
         }
-        rng_len[li] = overflow ? 0u : k;  // never let P2P read past the buffer
+        {
+            const RootC cc = leaf_centre(c_ctr, c, info + cell_system(c_sys, c));
+            LeafRec r{};
+            r.rng_off = base, r.rng_len = overflow ? 0u : k;  // never let P2P read past the buffer
+            r.src_total = src_total[li];
+            r.hx = cc.hx, r.hy = cc.hy, r.hz = cc.hz, r.lx = cc.lx, r.ly = cc.ly, r.lz = cc.lz;
+            leaf_rec[li] = r;
+        }
         const unsigned cb = chunk_off[li];
         const int nch = chunk_count(e - b);
-        const int ns = slice_count(src_total[li], slice);
+        const int ns = slice_count(src_total[li], leaf_slice(c, slice, fp32, n, seg, c_sys));
         for (int q = 0; q < nch; ++q) {
             int off, len;
             chunk_at(e - b, q, off, len);
@@ -1113,7 +1127,7 @@ void build_tree(Workspace &ws) {
                                 forest ? ws.c_sys : nullptr, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                                 reinterpret_cast<unsigned long long *>(&ws.info->m2l_pairs));
     k_rng_count<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
-                                    ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice);
+                                    ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, ws.mixed, n, seg, forest ? ws.c_sys : nullptr);
     {  // range, work-item and partial-slot offsets per leaf, one scan sequence
         ScanSet sc{};
         sc.in[0] = ws.rng_cnt, sc.out[0] = ws.rng_off, sc.total[0] = ws.d_counts + 4;
@@ -1122,8 +1136,8 @@ void build_tree(Workspace &ws) {
         scan_exclusive_multi(sc, 3, ws.c_cap, ws.d_counts + 3, ws.scan, st, &ws.launches);
     }
     k_rng_fill<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
-                                   ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.rng_len, ws.ranges, ws.chunk_off, ws.chunks,
-                                   ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice);
+                                   ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.leaf_rec, ws.c_ctr, ws.ranges, ws.chunk_off, ws.chunks,
+                                   ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, ws.mixed, n, seg, forest ? ws.c_sys : nullptr);
     ws.launches += 9;
     timer_end(ws, kTTree);
 }

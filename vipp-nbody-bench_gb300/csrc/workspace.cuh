@@ -29,6 +29,16 @@ namespace gb {
 
 enum TimerClass { kTTree = 0, kTOps = 1, kTUp = 2, kTM2L = 3, kTDown = 4, kTP2P = 5, kTRK4 = 6, kTSoft = 7, kNumTimers = 8 };
 
+// Near-field record of one leaf: its source ranges (after merging), their
+// sources, and its centre relative to the root-box centre as FP32 hi/lo parts
+// (RootC below). Written once per evaluation, so that a P2P work item finds it
+// in one read (and converts no FP64 centre: 15 operations on the narrow pipe).
+struct alignas(16) LeafRec {
+    unsigned rng_off, rng_len, src_total;
+    float hx, hy, hz, lx, ly, lz;
+    float pad_[3];
+};
+
 struct Workspace {
     // configuration of the evaluation
     int p = 4, K = 25, T = 90;  // T = floor(sqrt(8) s)
@@ -51,7 +61,6 @@ struct Workspace {
     // tuning knobs (gb_set_tuning / the tuning cache; the defaults are the measured best at 4M)
     unsigned p2p_blocks = 8;        // P2P blocks per SM when it runs alone (or after the far field)
     unsigned p2p_blocks_conc = 8;   // P2P blocks per SM launched beside the far field
-    int p2p_occ = 8;                // blocks per SM the mixed P2P kernel's registers are budgeted for (8 or 6)
     unsigned p2p_slice = kSliceSources;  // near-field sources per P2P work item
     int m2l_ctas_pct = 100;         // tensor-core M2L CTAs, percent of the SMs (one persistent CTA per SM)
 
@@ -130,7 +139,7 @@ struct Workspace {
     int *leaves = nullptr;            // [C]
     unsigned *rng_cnt = nullptr;      // [C] ranges per leaf before merging (then capacity offsets)
     unsigned *rng_off = nullptr;      // [C+1]
-    unsigned *rng_len = nullptr;      // [C] ranges per leaf after merging
+    LeafRec *leaf_rec = nullptr;      // [C] what a P2P work item reads of its leaf
     uint2 *ranges = nullptr;          // [r_cap]
     unsigned *chunk_cnt = nullptr, *chunk_off = nullptr;  // [C]
     int4 *chunks = nullptr;           // [ch_cap] work items (leaf, first target, packed sizes, partial slot)
