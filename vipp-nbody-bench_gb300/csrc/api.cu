@@ -293,6 +293,14 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
         }
     }
     if (ws.m2l_tensor) {
+        // part sums of small trees' tiles (or a scratch per CTA)
+        const unsigned tiles = std::min(gb::kM2LTcSplitTiles, gb::m2l_tc_tiles(ws));
+        if (tiles > ws.m2l_tc_tiles || ws.p > ws.m2l_tc_p) {
+            ++ctx->epoch;
+            GB_TRY(dalloc(ws.m2l_tc_part, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms))));
+            GB_TRY(dalloc(ws.m2l_tc_pcnt, tiles));
+            ws.m2l_tc_tiles = tiles, ws.m2l_tc_p = ws.p;
+        }
         // split expansions of the tensor-core M2L and their TMA map
         const int kp = gb::m2l_tc_row_floats(ws.p);
         const unsigned rows = ws.c_cap + gb::kZeroRows;
@@ -428,10 +436,20 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
     gb::Workspace &ws = ctx->ws;
     g_timer_ctx = ctx;
     gb::build_tree(ws);
+    if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : ws.mixed ? gb::kM2LTileCC : gb::kM2LTileF64);
     // Near field on the second stream, unless serial or timed: class timers
     // measure each class alone on one stream.
     const bool fork = !ws.serial && !ws.timing;
-    const unsigned conc = ws.p2p_blocks_conc, full = ws.p2p_blocks;
+    // Beside the far field, no more P2P blocks per SM than its tensor-core M2L leaves
+    // registers for (m2l_tc.cu): with more, the M2L's CTAs only
+    // start when the near field is done. Three against eight (then one after the
+    // other), ms per step: 4M Plummer 30.4 and 32.9, 16M clustered 126.0 and 133.8,
+    // 1M unit cube 5.7 and 6.3, 100,003 Plummer 3.00 and 3.40.
+    const unsigned full = ws.p2p_blocks;
+    // FP64: four (57,344 of the registers at eight leave the M2L none): 16,384
+    // Plummer 4.53 and 4.83, 262,144 unit cube 27.5 and 28.2.
+    const unsigned beside = !ws.mixed ? 4u : ws.m2l_tensor ? 3u : 16u;
+    const unsigned conc = std::min(ws.p2p_blocks_conc, beside);
     if (fork) {
         cudaEventRecord(ws.ev_fork, ws.st);
         cudaStreamWaitEvent(ws.st2, ws.ev_fork, 0);
@@ -453,7 +471,6 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
         cudaEventRecord(ws.ev_join3, ws.st3);
     }
     gb::build_operators(ws);
-    if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : ws.mixed ? gb::kM2LTileCC : gb::kM2LTileF64);
     gb::upward_pass(ws);
     if (ws.m2l_tensor)
         gb::m2l_pass_tc(ws);
@@ -741,7 +758,7 @@ void gb_destroy(gb_ctx *ctx) {
                     ws.split_cell, ws.c_begin, ws.c_end, ws.c_parent, ws.c_child, ws.c_level, ws.c_path, ws.c_coord,
                     ws.c_box, ws.c_ctr, ws.Mexp, ws.Lexp, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                     ws.flag, ws.flag_off, ws.leaves, ws.rng_cnt, ws.rng_off, ws.leaf_rec, ws.ranges, ws.chunk_cnt,
-                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.m2l_part, ws.m2l_pcnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
+                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.m2l_tc_part, ws.m2l_tc_pcnt, ws.m2l_part, ws.m2l_pcnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
                     ctx->d_direct, ws.seg, ws.psys, ws.c_sys, ws.sys_par, ws.mkeys, ws.etile, ws.oct_list, ws.otile,
                     ws.ocnt, ws.soft_corr};
     for (void *b : bufs) dfree(b);

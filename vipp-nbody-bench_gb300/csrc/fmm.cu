@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(256) k_m2l(const TreeInfo *__restrict__ info, 
 // writes the parents' multipoles. (One CTA doing the 8 octants in turn made a
 // level cost ~165 us whatever its size.)
 template <int P, typename T>
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, GB_FAR_MIN_BLOCKS)
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
     k_m2m(int L, const TreeInfo *__restrict__ info, const int *__restrict__ split_cell, const int *__restrict__ c_child,
           const T *__restrict__ ops_all, const int2 *__restrict__ etile, const int *__restrict__ c_sys, T *M) {
     namespace cg = cooperative_groups;
@@ -940,6 +940,7 @@ void launch_l2p_phi(Workspace &ws, double *farphi) {
 template <int P, typename T>
 void launch_p2m(Workspace &ws) {
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.c_cap, 4));
+    full_shared(k_p2m<P, T>);
     k_p2m<P, T><<<gs, 128, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_ctr, ws.xs, ws.ph,
                                        ws.pl, ws.n, ws.info, forest_cells(ws), ws.m, static_cast<T *>(ws.Mexp));
 }
@@ -947,6 +948,7 @@ void launch_p2m(Workspace &ws) {
 template <int P, typename T>
 void launch_l2p(Workspace &ws) {
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.c_cap, 4));
+    full_shared(k_l2p<P, T>);
     k_l2p<P, T><<<gs, 128, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_ctr, ws.xs, ws.ph,
                                        ws.pl, ws.n, ws.info, forest_cells(ws), static_cast<const T *>(ws.Lexp),
                                        static_cast<T *>(ws.farf));
@@ -961,6 +963,7 @@ template <int P, typename T>
 void launch_m2l(Workspace &ws) {
     const size_t smem = TileCfg<P, T>::smem;
     cudaFuncSetAttribute(k_m2l<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    full_shared(k_m2l<P, T>);
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2,
                                     8 * (ceil_div(ceil_div(ws.c_cap, 8), kTile) + (ws.forest() ? ws.nsys : 0)));
     k_m2l<P, T><<<gs, 256, smem, ws.st>>>(ws.info, ws.m2l_src, ops_of<P, T>(ws), ws.forest() ? ws.otile : nullptr,
@@ -972,6 +975,7 @@ template <int P, typename T>
 void launch_m2m_levels(Workspace &ws) {
     const size_t smem = TileCfg<P, T>::smem;
     cudaFuncSetAttribute(k_m2m<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    full_shared(k_m2m<P, T>);
     const unsigned gs = 8 * capped_grid(static_cast<unsigned>(ws.num_sms) / 8 * 2, ceil_div(ws.s_cap, kTile));  // clusters of 8 CTAs
     // no cell is deeper than the key levels the sort ordered (tree.cu), so
     // parents lie at levels < ws.sort_levels
@@ -986,6 +990,7 @@ template <int P, typename T>
 void launch_l2l_levels(Workspace &ws) {
     const size_t smem = TileCfg<P, T>::smem;
     cudaFuncSetAttribute(k_l2l<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    full_shared(k_l2l<P, T>);
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2, 8 * ceil_div(ws.s_cap, kTile));
     for (int Lp = 2; Lp <= ws.sort_levels - 1; ++Lp) {
         k_l2l<P, T><<<gs, 256, smem, ws.st>>>(Lp, ws.info, ws.split_cell, ws.c_child, ops_of<P, T>(ws),
@@ -1045,6 +1050,8 @@ void build_operators(Workspace &ws) {
         // M2L offsets: FP32 operators, kSysPerBlock systems per block; then M2M and L2L
         // few systems: a thread per order (latency); many: a thread per operator (FP64 work)
         const int cols = nsys < 16 ? 2 * ws.p + 1 : 1;
+        full_shared(k_zf_tables);
+        full_shared(k_build_ops_f);
         k_zf_tables<<<static_cast<unsigned>(ceil_div(static_cast<size_t>(nsys) * kNumOps * cols, 128)), 128, 0, ws.st>>>(
             ws.info, nsys, ws.p, cols, ws.zf);
         const size_t smem_f = kSysPerBlock * sizeof(float) * ny;
@@ -1052,6 +1059,7 @@ void build_operators(Workspace &ws) {
             nsys, ws.p, static_cast<const M2LEnt *>(ws.m2l_tab), ws.zf, ws.ops_f);
         ws.launches += 1;
     } else {
+        full_shared(k_build_ops);
         k_build_ops<<<dim3(kNumOps, nsys), 256, smem, ws.st>>>(ws.info, ws.p, static_cast<const M2LEnt *>(ws.m2l_tab), ws.ops_d,
                                                               ws.ops_f, false, 0);
     }

@@ -261,6 +261,7 @@ template <int P>
 void launch_m2l_f64(Workspace &ws) {
     constexpr size_t smem = static_cast<size_t>(kHRows) * kLanesF64 * sizeof(double);
     cudaFuncSetAttribute(k_m2l_f64<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    full_shared(k_m2l_f64<P>);
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2, static_cast<size_t>(m2l_f64_tiles(ws)) * kGroupsF64);
     k_m2l_f64<P><<<gs, kThreadsF64, smem, ws.st>>>(ws.info, ws.m2l_src, ws.ops_d, ws.forest() ? ws.otile : nullptr, ws.oct_list,
                                                    static_cast<const double *>(ws.Mexp), static_cast<double *>(ws.Lexp),

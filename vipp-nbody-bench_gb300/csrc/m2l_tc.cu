@@ -52,6 +52,14 @@
 // Every tile runs the same static schedule (189 slots x NKC chunks), so the
 // three roles agree on it without exchanging control data.
 //
+// A tile's sum is made of six parts of 32 slots, each summed on its own and the
+// parts added in order. A tree of fewer than kSplitTiles tiles runs each part as
+// a work unit of its own (one CTA per tile would leave most SMs idle: 24 tiles at
+// 100,000 particles), leaves the part in a buffer and the CTA that finishes a
+// tile's last part adds the six; larger trees run whole tiles and fold the parts
+// into a per-CTA scratch in the same order, so both give the same bits (a
+// forest's systems those of their own contexts).
+//
 // Every mbarrier wait is bounded by the global timer; on a timeout the CTA
 // records kDevTimeout in the status word, stops issuing work, waits (bounded)
 // for its own copies and MMAs, frees its TMEM and returns.
@@ -70,38 +78,16 @@ constexpr int kRows = 128;          // targets per tile (MMA M)
 static_assert(kRows == kM2LTileTC, "forest M2L tiles");
 constexpr int kKC32 = 32;           // K chunk in 4-byte units: one 128-byte swizzle row
 constexpr int kDrainThreads = 128;  // warps 0-3
-#ifndef M2L_LOADER_WARPS
-#define M2L_LOADER_WARPS 4
-#endif
-#ifndef M2L_MAX_STAGES
-#define M2L_MAX_STAGES 4  // tf32 stages (56 KB each)
-#endif
-#ifndef M2L_MAX_STAGES_BF16
-#define M2L_MAX_STAGES_BF16 5  // bf16 stages (40 KB each)
-#endif
-#ifndef M2L_MIN_BLOCKS
-#define M2L_MIN_BLOCKS 1  // > 1 caps registers so the kernel fits beside P2P blocks
-#endif
-#ifndef M2L_WIDE_B
-#define M2L_WIDE_B 1
-#endif
-#ifndef M2L_TMEM_TOTAL
-#define M2L_TMEM_TOTAL 1  // drain keeps a tile's running sums in free TMEM columns, not registers
-#endif
-constexpr int kLoaderWarps = M2L_LOADER_WARPS;  // warps 4 .. 3 + kLoaderWarps
-constexpr int kMmaWarp = 4 + kLoaderWarps;
-constexpr int kThreads = 32 * (kMmaWarp + 1);
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s per wait
-#ifndef M2L_PREFETCH2
-#define M2L_PREFETCH2 1  // source rows of two slots ahead in flight instead of one (~1% faster at 4M)
-#endif
-#ifndef M2L_GROUP
-#define M2L_GROUP 4
-#endif
-constexpr int kGroup = M2L_GROUP;   // slots per TMEM accumulation group
+constexpr int kGroup = 4;           // slots per TMEM accumulation group
 constexpr int kSlotsPerTile = 189;  // M2L slots of every octant: 216 minus the 27 adjacent ones
 constexpr int kGroupsPerTile = (kSlotsPerTile + kGroup - 1) / kGroup;
+constexpr int kPartSlots = 32;      // slots per part of a tile's sum
+constexpr int kParts = (kSlotsPerTile + kPartSlots - 1) / kPartSlots;
+constexpr int kPartGroups = kPartSlots / kGroup;
+static_assert(kPartSlots % kGroup == 0, "parts of whole groups");
 constexpr int kSmemMax = 232448;    // opt-in shared memory per block
+constexpr int kSmemBeside = kSmemMax - 4 * 4352;  // what four P2P blocks leave of an SM's
 
 template <int P, bool BF>
 struct TcCfg {
@@ -116,14 +102,14 @@ struct TcCfg {
     static constexpr int N = (K + 15) / 16 * 16;         // MMA N (multiple of 16 for M = 128)
     // An accumulator holds A [Bhi; Blo]^T (2N columns; the two halves are added
     // by the drain), so the hi and lo operator blocks are adjacent in the stage.
-    static constexpr int DCOLS = (BF || M2L_WIDE_B) ? 2 * N : N;
+    static constexpr int DCOLS = 2 * N;
     static constexpr int ACOL = DCOLS <= 32 ? 32 : (DCOLS <= 64 ? 64 : (DCOLS <= 128 ? 128 : 256));
-    // The tile's running sums (NCH chunks of 32 columns) stay in TMEM when
+    // A part's running sums (NCH chunks of 32 columns) stay in TMEM when
     // columns are free: after both accumulators, or in the gaps behind them.
     static constexpr int NCH = (N + 31) / 32;
     static constexpr bool TOT_AFTER = 2 * ACOL + 32 * NCH <= 512;
     static constexpr int GAPCH = (ACOL - DCOLS) / 32;
-    static constexpr bool TOTAL_TMEM = M2L_TMEM_TOTAL && (TOT_AFTER || 2 * GAPCH >= NCH);
+    static constexpr bool TOTAL_TMEM = TOT_AFTER || 2 * GAPCH >= NCH;  // p <= 8
     static constexpr int TMEM_COLS = TOTAL_TMEM ? 512 : 2 * ACOL;
     static constexpr uint32_t tcol(int k) {
         return static_cast<uint32_t>(TOT_AFTER ? 2 * ACOL + 32 * k : (k < GAPCH ? DCOLS + 32 * k : ACOL + DCOLS + 32 * (k - GAPCH)));
@@ -131,9 +117,28 @@ struct TcCfg {
     static constexpr int A_BYTES = kRows * 128;          // one A tile: 16 KB
     static constexpr int B_BYTES = N * 128;              // one of Bhi / Blo
     static constexpr int STAGE = NA * A_BYTES + 2 * B_BYTES;
-    static constexpr int MAX_STAGES = BF ? M2L_MAX_STAGES_BF16 : M2L_MAX_STAGES;
-    static constexpr int STAGES = (kSmemMax - 2048) / STAGE >= MAX_STAGES ? MAX_STAGES : (kSmemMax - 2048) / STAGE;  // ring depth
-    static constexpr size_t SMEM = static_cast<size_t>(STAGES) * STAGE + 1024 + 256;
+    // Three stages: two to five measured the same (the copies of a step take
+    // longer to post than to arrive), and the rest of the shared memory holds the
+    // tile's sum (SUM_SMEM) and leaves room for P2P blocks.
+    // (two cost 27% at p = 8, bf16; at p >= 9, tf32 their 60 KB stages are two.)
+    static constexpr int STAGES = !TOTAL_TMEM && !BF ? 2 : 3;
+    // Loader warps: posting a gather4 takes a warp ~150 cycles (its operands go
+    // through uniform registers lane by lane), so eight warps post a step's copies
+    // faster than four (4M particles, p = 8, bf16: 1.60 -> 1.37 ms per evaluation;
+    // 16 warps 1.39).
+    static constexpr int LOADERS = 8;
+    static constexpr int MMA_WARP = 4 + LOADERS;
+    static constexpr int THREADS = 32 * (MMA_WARP + 1);
+    // 64 registers, so that three P2P blocks (80 registers, one warp per scheduler
+    // each) fit beside this kernel's four warps on a scheduler
+    static constexpr int BOUND_THREADS = 512;
+    static constexpr int BOUND_BLOCKS = 2;
+    // Shared memory [coefficient][row]: the part's running sums where TMEM has no
+    // columns for them (p >= 9), else the tile's sum where it fits
+    static constexpr int SUM_BYTES = K * kRows * 4;
+    static constexpr bool SUM_SMEM = STAGES * STAGE + SUM_BYTES + 1280 <= kSmemBeside;
+    static_assert(TOTAL_TMEM || SUM_SMEM, "running sums");
+    static constexpr size_t SMEM = static_cast<size_t>(STAGES) * STAGE + (SUM_SMEM ? SUM_BYTES : 0) + 1024 + 256;
     // instruction descriptor: D f32 (bits 4-5 = 1), A/B bf16 (bits 7-9, 10-12 = 1,
     // kind::f16) or tf32 (= 2, kind::tf32), both K-major, N >> 3 at bits 17-22,
     // M >> 4 at bits 24-28
@@ -144,8 +149,7 @@ struct TcCfg {
     static constexpr uint32_t IDESC = idesc(N);
     static constexpr uint32_t IDESC_W = idesc(2 * N);
     static_assert(2 * N <= 256, "MMA N");
-    static_assert(STAGES >= 3, "ring depth");
-    static_assert(GATHERS % kLoaderWarps == 0, "loader warps");
+    static_assert(GATHERS % LOADERS == 0, "loader warps");
     static_assert(STAGE % 1024 == 0, "stages must keep the 1024-byte swizzle atoms aligned");
     static_assert(SMEM <= static_cast<size_t>(kSmemMax), "shared memory");
 };
@@ -242,41 +246,44 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar)) : "memory");
 }
 
+// Barrier of the four drain warps; whether any of their threads passed true.
+__device__ __forceinline__ bool drain_or(int v) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r)
+                 : "r"(v), "n"(kDrainThreads)
+                 : "memory");
+    return r != 0;
+}
+
 __device__ __forceinline__ float tf32_hi(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
-    uint32_t r[32];
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
+    uint32_t r[16];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float *v) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *v) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(
+            taddr),
         "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
         "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
         "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
-        "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-        "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-        "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
-        "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
+        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
         : "memory");
 }
 
 // Slot s of a target with octant cls maps to same-level offset 2d + u(o') - u(cls);
 // adjacent offsets are not M2L slots. Returns the operator index or -1.
-__host__ __device__ __forceinline__ int slot_operator(int cls, int s) {
+__host__ __device__ constexpr int slot_operator(int cls, int s) {
     const int dd = s >> 3, o = s & 7;
     const int uc0 = 1 - (cls & 1), uc1 = 1 - ((cls >> 1) & 1), uc2 = 1 - ((cls >> 2) & 1);
     const int o0 = 2 * (dd % 3 - 1) + 1 - (o & 1) - uc0;
@@ -286,10 +293,20 @@ __host__ __device__ __forceinline__ int slot_operator(int cls, int s) {
     return (o0 + 3) + 7 * (o1 + 3) + 49 * (o2 + 3);
 }
 
-__device__ __forceinline__ int next_slot(int cls, int s) {
-    while (s < kM2LSlots && slot_operator(cls, s) < 0) ++s;
-    return s;
+// The 189 M2L slots of each octant, in order.
+struct SlotTab {
+    unsigned char s[8][kSlotsPerTile];
+};
+constexpr SlotTab slot_table() {
+    SlotTab t{};
+    for (int cls = 0; cls < 8; ++cls) {
+        int n = 0;
+        for (int s = 0; s < kM2LSlots; ++s)
+            if (slot_operator(cls, s) >= 0) t.s[cls][n++] = static_cast<unsigned char>(s);
+    }
+    return t;
 }
+__constant__ SlotTab c_slots = slot_table();
 
 // Target cell of row r of tile-job w (octant w % 8, tile w / 8), or -1: one
 // tree's tiles take consecutive octets; a forest's take its per-system octet
@@ -305,20 +322,23 @@ __device__ __forceinline__ int tc_row_cell(int w, int r, int base, int per_class
 }
 
 template <int P, bool BF>
-__global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
+__global__ void __launch_bounds__((TcCfg<P, BF>::BOUND_THREADS), (TcCfg<P, BF>::BOUND_BLOCKS))
     k_m2l_tc(const __grid_constant__ CUtensorMap tmap, const TreeInfo *__restrict__ info, const int *__restrict__ m2l_src,
              const unsigned char *__restrict__ bimg_all, const int4 *__restrict__ otile, const int *__restrict__ oct_list,
-             int rows_cap, float *__restrict__ Lx, TreeInfo *info_rw) {
+             int rows_cap, float *__restrict__ Lx, TreeInfo *info_rw, float *__restrict__ part, unsigned *pcnt, int split_tiles) {
     using C = TcCfg<P, BF>;
-    constexpr int kGW = C::GATHERS / kLoaderWarps;  // gather4 copies per loader warp and step
+    constexpr int kGW = C::GATHERS / C::LOADERS;  // gather4 copies per loader warp and step
+    constexpr int kMmaWarp = C::MMA_WARP;
     extern __shared__ __align__(1024) unsigned char sm_raw[];
     unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(sm + C::STAGES * C::STAGE);
+    float *sums = reinterpret_cast<float *>(sm + C::STAGES * C::STAGE);  // [K][row], SUM_SMEM
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + C::STAGES * C::STAGE + (C::SUM_SMEM ? C::SUM_BYTES : 0));
     uint64_t *empty = full + C::STAGES;
     uint64_t *accum = empty + C::STAGES;  // [2]: group finished in accumulator a
     uint64_t *tfree = accum + 2;        // [2]: accumulator a drained
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tfree + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *last_flag = abort_flag + 1;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int base = info->level_start[2];
@@ -326,10 +346,13 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
     const int per_class = ntgt > 0 ? ntgt / 8 : 0;
     const int tiles_per_class = otile ? info->n_otiles : (per_class + kRows - 1) / kRows;
     const int ntiles = ntgt > 0 ? 8 * tiles_per_class : 0;
-    if (ntiles == 0 || static_cast<int>(blockIdx.x) >= ntiles) return;  // uniform: no barrier or TMEM touched yet
+    // work units: tiles (parts 0 .. kParts-1 in turn), or one part of a tile each
+    const bool split = ntiles <= split_tiles;
+    const int units = split ? kParts * ntiles : ntiles;
+    if (static_cast<int>(blockIdx.x) >= units) return;  // uniform: no barrier or TMEM touched yet
 
     if (tid == 0) {
-        for (int s = 0; s < C::STAGES; ++s) mbar_init(full + s, kLoaderWarps), mbar_init(empty + s, 1);
+        for (int s = 0; s < C::STAGES; ++s) mbar_init(full + s, C::LOADERS), mbar_init(empty + s, 1);
         for (int a = 0; a < 2; ++a) mbar_init(accum + a, 1), mbar_init(tfree + a, kDrainThreads);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -366,8 +389,9 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
         const int zrow = rows_cap - kZeroRows + quad;
         unsigned step = 0;
         bool stop = false;
-        for (int w = blockIdx.x; w < ntiles && !stop; w += gridDim.x) {
-            const int cls = w % 8;
+        for (int unit = blockIdx.x; unit < units && !stop; unit += gridDim.x) {
+            const int w = split ? unit % ntiles : unit, cls = w % 8;
+            const int j0 = split ? unit / ntiles * kPartSlots : 0, j1 = split ? min(kSlotsPerTile, j0 + kPartSlots) : kSlotsPerTile;
             // a forest tile's operator images are its system's
             const unsigned char *bimg =
                 otile ? bimg_all + static_cast<size_t>(otile[w / 8].x) * (kNumOffsets * C::NKC * 2 * C::B_BYTES) : bimg_all;
@@ -388,27 +412,15 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
                     r[i] = src >= 0 ? src : zrow;
                 }
             };
-            int s = next_slot(cls, 0);
-            int cur[4];
-            rows_of(s, cur);
-#if M2L_PREFETCH2
-            // source rows two slots ahead: the loads of slot s + 2 are in flight
-            // while slots s and s + 1 are posted
-            int sn = s < kM2LSlots ? next_slot(cls, s + 1) : kM2LSlots;
-            int nxt[4] = {zrow, zrow, zrow, zrow};
-            if (sn < kM2LSlots) rows_of(sn, nxt);
-            while (s < kM2LSlots && !stop) {
-                const int oi = slot_operator(cls, s);
-                const int snn = sn < kM2LSlots ? next_slot(cls, sn + 1) : kM2LSlots;
+            // source rows two slots ahead: the loads of slot j + 2 are in flight
+            // while slots j and j + 1 are posted (~1% faster at 4M than one ahead)
+            int cur[4], nxt[4] = {zrow, zrow, zrow, zrow};
+            rows_of(c_slots.s[cls][j0], cur);
+            if (j0 + 1 < j1) rows_of(c_slots.s[cls][j0 + 1], nxt);
+            for (int j = j0; j < j1 && !stop; ++j) {
+                const int oi = slot_operator(cls, c_slots.s[cls][j]);
                 int nxt2[4] = {zrow, zrow, zrow, zrow};
-                if (snn < kM2LSlots) rows_of(snn, nxt2);
-#else
-            while (s < kM2LSlots && !stop) {
-                const int oi = slot_operator(cls, s);
-                const int sn = next_slot(cls, s + 1);
-                int nxt[4] = {zrow, zrow, zrow, zrow};
-                if (sn < kM2LSlots) rows_of(sn, nxt);  // in flight while this slot's copies are posted
-#endif
+                if (j + 2 < j1) rows_of(c_slots.s[cls][j + 2], nxt2);
                 for (int kc = 0; kc < C::NKC; ++kc, ++step) {
                     const int st = step % C::STAGES;
                     const unsigned use = step / C::STAGES;
@@ -431,16 +443,8 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
                         bulk_g2s(stage + C::NA * C::A_BYTES, bimg + (static_cast<size_t>(oi) * C::NKC + kc) * (2 * C::B_BYTES),
                                  b_bytes(kc), full + st);
                 }
-#if M2L_PREFETCH2
 #pragma unroll
                 for (int i = 0; i < 4; ++i) cur[i] = nxt[i], nxt[i] = nxt2[i];
-                s = sn;
-                sn = snn;
-#else
-#pragma unroll
-                for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
-                s = sn;
-#endif
             }
         }
     } else if (warp == kMmaWarp) {
@@ -448,8 +452,9 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
         if (lane == 0) {
             unsigned groups = 0;
             bool stop = false;
-            for (int w = blockIdx.x; w < ntiles && !stop; w += gridDim.x) {
-                for (int j = 0; j < kSlotsPerTile && !stop; ++j) {
+            for (int unit = blockIdx.x; unit < units && !stop; unit += gridDim.x) {
+                const int j0 = split ? unit / ntiles * kPartSlots : 0, j1 = split ? min(kSlotsPerTile, j0 + kPartSlots) : kSlotsPerTile;
+                for (int j = j0; j < j1 && !stop; ++j) {
                     const int in_group = j % kGroup;
                     const unsigned a = groups & 1;
                     // a group reuses accumulator a once group - 2 has been drained
@@ -469,7 +474,6 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
                         const unsigned char *stage = sm + st * C::STAGE;
                         const uint64_t ahi = sdesc_sw128(stage);
                         const unsigned char *Bhi = stage + C::NA * C::A_BYTES;
-                        const unsigned char *Blo = Bhi + C::B_BYTES;
                         const int ksteps = min(C::KC / C::KS, (C::KA - kc * C::KC + C::KS - 1) / C::KS);
                         for (int ks = 0; ks < ksteps; ++ks) {
                             // 32 B along K: +2 in the swizzled start field, two
@@ -483,12 +487,7 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
                                 umma_bf16(dt, ahi + 2 * ks, bhi, wide ? C::IDESC_W : C::IDESC, first);
                             } else {
                                 const uint64_t alo = sdesc_sw128(stage + C::A_BYTES);
-                                if (M2L_WIDE_B) {
-                                    umma_tf32(dt, ahi + 2 * ks, bhi, C::IDESC_W, first);  // Ahi [Bhi; Blo]^T
-                                } else {
-                                    umma_tf32(dt, ahi + 2 * ks, bhi, C::IDESC, first);
-                                    umma_tf32(dt, ahi + 2 * ks, sdesc(Blo + ks * 256), C::IDESC, 1u);
-                                }
+                                umma_tf32(dt, ahi + 2 * ks, bhi, C::IDESC_W, first);  // Ahi [Bhi; Blo]^T
                                 umma_tf32(dt, alo + 2 * ks, bhi, C::IDESC, 1u);
                             }
                         }
@@ -496,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
                         ++mma_steps;
                     }
                     if (stop) break;
-                    if (in_group == kGroup - 1 || j == kSlotsPerTile - 1) {
+                    if (in_group == kGroup - 1 || j == j1 - 1) {
                         umma_commit(accum + a);
                         ++groups;
                     }
@@ -509,82 +508,107 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
         unsigned groups = 0;
         bool stop = false;
         const uint32_t lanes = tmem + (static_cast<uint32_t>(32 * warp) << 16);  // TMEM lanes 32 warp .. + 31
-        if (C::TOTAL_TMEM) {
-            // running sums in TMEM (columns tcol(k)), added in the same order as
-            // the register form below: total, then each half of the group
-            for (int w = blockIdx.x; w < ntiles && !stop; w += gridDim.x) {
-                for (int gi = 0; gi < kGroupsPerTile; ++gi, ++groups) {
+        constexpr size_t kPartFloats = static_cast<size_t>(C::N) * kRows;        // [column][row]
+        for (int unit = blockIdx.x; unit < units && !stop; unit += gridDim.x) {
+            const int w = split ? unit % ntiles : unit;
+            const int p0 = split ? unit / ntiles : 0, p1 = split ? p0 + 1 : kParts;
+            const int cell = tc_row_cell(w, tid, base, per_class, otile, oct_list);
+            float *out = Lx + static_cast<size_t>(cell < 0 ? 0 : cell) * C::K;
+            float *buf = part + (split ? static_cast<size_t>(w) * kParts + p0 : static_cast<size_t>(blockIdx.x)) * kPartFloats + tid;
+            for (int pt = p0; pt < p1 && !stop; ++pt) {
+                const int ng = min(kPartGroups, kGroupsPerTile - pt * kPartGroups);
+                for (int gi = 0; gi < ng; ++gi, ++groups) {
                     if (!__all_sync(0xffffffffu, mbar_wait(accum + (groups & 1), (groups >> 1) & 1, abort_flag))) {
                         stop = true;
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t col = (groups & 1) * C::ACOL;
+                    // sum, then each half of the group, 16 columns at a time
 #pragma unroll 1
-                    for (int k = 0; k < C::NCH; ++k) {
-                        float sum[32], v[32];
-                        if (gi > 0) {
-                            tmem_ld32(lanes + C::tcol(k), sum);
+                    for (int k = 0; k < C::N / 16; ++k) {
+                        const uint32_t tc = lanes + C::tcol(k >> 1) + 16 * (k & 1);
+                        float *sm_sum = sums + 16 * k * kRows + tid;
+                        float sum[16], v[16];
+                        if (gi == 0) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) sum[i] = 0.f;
+                        } else if constexpr (C::TOTAL_TMEM) {
+                            tmem_ld16(tc, sum);
                         } else {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+                            for (int i = 0; i < 16; ++i) sum[i] = 16 * k + i < C::K ? sm_sum[i * kRows] : 0.f;
                         }
 #pragma unroll
-                        for (int h = 0; h < C::DCOLS / C::N; ++h) {
-                            tmem_ld32(lanes + col + static_cast<uint32_t>(h * C::N + 32 * k), v);
+                        for (int h = 0; h < 2; ++h) {
+                            tmem_ld16(lanes + col + static_cast<uint32_t>(h * C::N + 16 * k), v);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) sum[i] += v[i];
+                            for (int i = 0; i < 16; ++i) sum[i] += v[i];
                         }
-                        tmem_st32(lanes + C::tcol(k), sum);
+                        if constexpr (C::TOTAL_TMEM) {
+                            tmem_st16(tc, sum);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if (16 * k + i < C::K) sm_sum[i * kRows] = sum[i];
+                        }
                     }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    if constexpr (C::TOTAL_TMEM) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     mbar_arrive(tfree + (groups & 1));
                 }
                 if (stop) break;
-                const int cell = tc_row_cell(w, tid, base, per_class, otile, oct_list);
-                float *out = Lx + static_cast<size_t>(cell < 0 ? 0 : cell) * C::K;
+                // the part is complete: into the buffer, or folded into the tile's sum
+                constexpr bool kTileSumSmem = C::TOTAL_TMEM && C::SUM_SMEM;
+                auto store = [&](int c, float v) {
+                    float *ts = kTileSumSmem ? sums + c * kRows + tid : buf + c * kRows;
+                    if (!split && pt > 0) v = (kTileSumSmem ? *ts : __ldcg(ts)) + v;
+                    if (split)
+                        __stcg(buf + c * kRows, v);
+                    else if (pt == kParts - 1) {
+                        if (cell >= 0) out[c] = v;
+                    } else if (kTileSumSmem)
+                        *ts = v;
+                    else
+                        __stcg(ts, v);
+                };
 #pragma unroll 1
-                for (int k = 0; k < C::NCH; ++k) {
-                    float sum[32];
-                    tmem_ld32(lanes + C::tcol(k), sum);  // all lanes: the load is warp-collective
+                for (int k = 0; k < C::N / 16; ++k) {
+                    float sum[16];
+                    if constexpr (C::TOTAL_TMEM) {
+                        tmem_ld16(lanes + C::tcol(k >> 1) + 16 * (k & 1), sum);  // all lanes: the load is warp-collective
+                    } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (cell >= 0 && 32 * k + i < C::K) out[32 * k + i] = sum[i];
+                        for (int i = 0; i < 16; ++i) sum[i] = 16 * k + i < C::K ? sums[(16 * k + i) * kRows + tid] : 0.f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (16 * k + i < C::K) store(16 * k + i, sum[i]);
                 }
             }
-        } else {
-        float acc[C::N];
-        for (int w = blockIdx.x; w < ntiles && !stop; w += gridDim.x) {
-#pragma unroll
-            for (int i = 0; i < C::N; ++i) acc[i] = 0.f;
-            for (int gi = 0; gi < kGroupsPerTile; ++gi, ++groups) {
-                if (!__all_sync(0xffffffffu, mbar_wait(accum + (groups & 1), (groups >> 1) & 1, abort_flag))) {
+            if (split) {
+                // every drain warp comes here once per unit, whatever its waits said: they
+                // agree on stopping, so none is left at a barrier
+                __threadfence();
+                if (drain_or(stop)) {
                     stop = true;
                     break;
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t col = (groups & 1) * C::ACOL;
+                // the last part of a tile to finish adds the parts in order
+                if (tid == 0) *last_flag = atomicAdd(pcnt + w, 1u) == kParts - 1;
+                drain_or(0);
+                if (*last_flag && cell >= 0) {
+                    __threadfence();
+                    const float *q = part + static_cast<size_t>(w) * kParts * kPartFloats + tid;
+                    for (int c = 0; c < C::K; ++c) {
+                        float v = __ldcg(q + c * kRows);
 #pragma unroll
-                for (int h = 0; h < C::DCOLS / C::N; ++h)
-#pragma unroll
-                    for (int c0 = 0; c0 < C::N; c0 += 32) {
-                        float v[32];
-                        tmem_ld32(tmem + (static_cast<uint32_t>(32 * warp) << 16) + col + static_cast<uint32_t>(h * C::N + c0), v);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (c0 + i < C::N) acc[c0 + i] += v[i];
+                        for (int pt = 1; pt < kParts; ++pt) v += __ldcg(q + pt * kPartFloats + c * kRows);
+                        out[c] = v;
                     }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(tfree + (groups & 1));
+                }
+                drain_or(0);  // last_flag is read
             }
-            if (stop) break;
-            const int cell = tc_row_cell(w, tid, base, per_class, otile, oct_list);
-            if (cell >= 0) {
-                float *out = Lx + static_cast<size_t>(cell) * C::K;
-                for (int r = 0; r < C::K; ++r) out[r] = acc[r];
-            }
-        }
         }
     }
     // Orderly exit: every wait above is bounded, so all threads get here.
@@ -614,8 +638,11 @@ __global__ void __launch_bounds__(kThreads, M2L_MIN_BLOCKS)
 // tf32: rows [0, rows_cap) hold the hi parts, rows [rows_cap, 2 rows_cap) the
 // lo parts, KP floats each, zero beyond K.
 template <int P, bool BF>
-__global__ void k_split_m(const TreeInfo *__restrict__ info, const float *__restrict__ M, void *__restrict__ ms_v, int rows_cap) {
+__global__ void k_split_m(const TreeInfo *__restrict__ info, const float *__restrict__ M, void *__restrict__ ms_v, int rows_cap,
+                          unsigned *pcnt, int tiles) {
     using C = TcCfg<P, BF>;
+    if (blockIdx.x == 0)  // no part of any tile is finished
+        for (int t = threadIdx.x; t < tiles; t += blockDim.x) pcnt[t] = 0;
     const int nc = min(info->ncells, rows_cap - kZeroRows);
     const size_t total = static_cast<size_t>(nc) * C::KP;
     const size_t zrow = static_cast<size_t>(rows_cap - kZeroRows) * C::KP;
@@ -723,17 +750,22 @@ void launch(Workspace &ws) {
     const int op_smem = static_cast<int>(sizeof(float) * C::K * C::K);
     if (op_smem > 48 * 1024)
         cudaFuncSetAttribute(k_build_bimg<P, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, op_smem);
+    full_shared(k_build_bimg<P, BF>);
+    full_shared(k_split_m<P, BF>);
+    full_shared(k_m2l_tc<P, BF>);
     k_build_bimg<P, BF><<<dim3(kNumOffsets, forest ? ws.nsys : 1), 256, op_smem, ws.st>>>(ws.ops_f,
                                                                                  reinterpret_cast<unsigned char *>(ws.bimg));
     k_split_m<P, BF><<<4 * ws.num_sms, 256, 0, ws.st>>>(ws.info, static_cast<const float *>(ws.Mexp), ws.ms_tc,
-                                                        static_cast<int>(ws.ms_rows));
+                                                        static_cast<int>(ws.ms_rows), ws.m2l_tc_pcnt,
+                                                        static_cast<int>(ws.m2l_tc_tiles));
     cudaFuncSetAttribute(k_m2l_tc<P, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C::SMEM));
     const unsigned ctas = std::max(1u, static_cast<unsigned>(ws.num_sms * ws.m2l_ctas_pct / 100));
-    const unsigned gs = capped_grid(ctas, 8 * (ceil_div(ceil_div(ws.c_cap, 8), kRows) + (forest ? ws.nsys : 0)));  // tiles
-    k_m2l_tc<P, BF><<<gs, kThreads, C::SMEM, ws.st>>>(ws.tmap_ms, ws.info, ws.m2l_src,
+    const unsigned gs = capped_grid(ctas, static_cast<size_t>(m2l_tc_tiles(ws)) * kParts);
+    k_m2l_tc<P, BF><<<gs, C::THREADS, C::SMEM, ws.st>>>(ws.tmap_ms, ws.info, ws.m2l_src,
                                                       reinterpret_cast<const unsigned char *>(ws.bimg),
                                                       forest ? ws.otile : nullptr, ws.oct_list,
-                                                      static_cast<int>(ws.ms_rows), static_cast<float *>(ws.Lexp), ws.info);
+                                                      static_cast<int>(ws.ms_rows), static_cast<float *>(ws.Lexp), ws.info,
+                                                      ws.m2l_tc_part, ws.m2l_tc_pcnt, static_cast<int>(ws.m2l_tc_tiles));
     ws.launches += 3;
 }
 
@@ -764,6 +796,15 @@ size_t m2l_tc_image_floats(int p) {
 int m2l_tc_row_floats(int p) {
     const int K = (p + 1) * (p + 1);
     return (K + kKC32 - 1) / kKC32 * kKC32;
+}
+
+unsigned m2l_tc_tiles(const Workspace &ws) {
+    return 8 * static_cast<unsigned>(ceil_div(ceil_div(ws.c_cap, 8), kRows) + (ws.forest() ? ws.nsys : 0));
+}
+// part sums of `tiles` split tiles, and at least one scratch per CTA
+size_t m2l_tc_part_floats(int p, unsigned tiles, unsigned ctas) {
+    const size_t N = static_cast<size_t>((p + 1) * (p + 1) + 15) / 16 * 16;
+    return N * kRows * std::max<size_t>(static_cast<size_t>(tiles) * kParts, ctas);
 }
 
 bool m2l_tc_supported(int p) { return p >= 2 && p <= kMaxP; }

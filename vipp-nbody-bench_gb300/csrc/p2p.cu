@@ -25,10 +25,6 @@
 #include "rinv.cuh"
 #include "workspace.cuh"
 
-#ifndef GB_P2P_CARVEOUT_MAX
-#define GB_P2P_CARVEOUT_MAX 1  // P2P SMs keep full shared memory, so the tensor-core M2L can start beside P2P blocks
-#endif
-
 namespace gb {
 
 namespace {
@@ -454,21 +450,9 @@ void near_potential(Workspace &ws, double *phiv) {
 // launches (on any streams) may drain the same queue, each item is taken once.
 // p2p_finish adds the slices of split items after all of them.
 
-void p2p_f32_carveout() {
-    // keep the SMs that run P2P configured for full shared memory, so far-field
-    // kernels (the tensor-core M2L: up to 206 KB) can start beside the P2P blocks
-    cudaFuncSetAttribute(k_p2p_f32<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<true, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_p2p_f32<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-}
-
 void p2p_pass(Workspace &ws, unsigned per_sm) {
     if (per_sm == 0) return;
     timer_begin(ws, kTP2P);
-#if GB_P2P_CARVEOUT_MAX
-    p2p_f32_carveout();
-#endif
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * per_sm, ceil_div(ws.ch_cap, kP2PWarps));
     const bool soft = ws.eps > 0;
     if (ws.mixed) {
@@ -477,18 +461,17 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
         auto *o = static_cast<float *>(ws.nearf);
         auto *pf = static_cast<float *>(ws.part);
 #define GB_P2P32(NW, SF)                                                                                             \
+    full_shared(k_p2p_f32<NW, SF>);                                                                                  \
     k_p2p_f32<NW, SF><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.ph, \
                                                         ws.pl, pf, Gm, eps2, o, ws.n)
-        if (ws.p2p_newton) {
-            if (soft)
-                GB_P2P32(true, true);
-            else
-                GB_P2P32(true, false);
+        if (ws.p2p_newton && soft) {
+            GB_P2P32(true, true);
+        } else if (ws.p2p_newton) {
+            GB_P2P32(true, false);
+        } else if (soft) {
+            GB_P2P32(false, true);
         } else {
-            if (soft)
-                GB_P2P32(false, true);
-            else
-                GB_P2P32(false, false);
+            GB_P2P32(false, false);
         }
 #undef GB_P2P32
     } else {
@@ -496,6 +479,8 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
         auto *o = static_cast<double *>(ws.nearf);
         auto *pd = static_cast<double *>(ws.part);
         const SoftInt si = soft_int(eps2);
+        full_shared(k_p2p_f64<true>);
+        full_shared(k_p2p_f64<false>);
         if (soft)
             k_p2p_f64<true><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges,
                                                               ws.xs, pd, Gm, eps2, si, o, ws.n);

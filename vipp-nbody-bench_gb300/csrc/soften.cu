@@ -658,6 +658,10 @@ void launch_soften(Workspace &ws, T *corr) {
     T *taylor = static_cast<T *>(ws.staylor);
     const T e2 = static_cast<T>(ws.eps * ws.eps);
     if (corr) cudaMemsetAsync(corr, 0, sizeof(T) * 3 * static_cast<size_t>(ws.n), ws.st);
+    full_shared(k_mom_leaf<T>);
+    full_shared(k_mom_up<T>);
+    full_shared(k_soft_far<T>);
+    full_shared(k_soft_near<T>);
     k_mom_leaf<T><<<gw, 128, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_ctr, ws.xs, ws.ph,
                                          ws.pl, ws.n, ws.info, static_cast<T>(ws.m), mom, moct);
     ws.launches += 1;

@@ -161,6 +161,10 @@ struct Workspace {
     bool ms_bf16 = false;     // the split form tmap_ms was encoded for
     CUtensorMap tmap_ms{};    // TMA map of ms_tc
 
+    float *m2l_tc_part = nullptr;    // tensor-core M2L: part sums of small trees' tiles, or a scratch per CTA (m2l_tc.cu)
+    unsigned *m2l_tc_pcnt = nullptr; // [m2l_tc_tiles] finished parts of a tile (zeroed by k_split_m)
+    unsigned m2l_tc_tiles = 0;       // tiles the two are sized for
+    int m2l_tc_p = 0;                // and the expansion order
     double *m2l_part = nullptr;   // FP64 M2L: class-group sums of small trees' tiles (m2l_fp64.cu)
     unsigned *m2l_pcnt = nullptr; // [m2l_part_tiles] finished groups of a tile, zero between evaluations
     unsigned m2l_part_tiles = 0;  // tiles the two are sized for
@@ -198,6 +202,9 @@ constexpr int kM2LTileTC = 128;  // target octets per tensor-core M2L tile (m2l_
 constexpr int kZeroRows = 32;    // zero rows after the split expansions (one per row quad of a tile)
 constexpr int kM2LTileCC = 64;   // per FP32 CUDA-core M2L tile (fmm.cu)
 constexpr int kM2LTileF64 = 32;  // per FP64 M2L tile (m2l_fp64.cu)
+// Tensor-core M2L tiles up to which their parts run as units of their own: two
+// rounds of one CTA per SM (beyond that whole tiles fill the SMs)
+constexpr unsigned kM2LTcSplitTiles = 304;
 // FP64 M2L tiles (32 targets of one octant) up to which a tile's class groups
 // run as blocks of their own: two blocks on each of the 152 SMs
 constexpr unsigned kM2LSplitTiles = 304;
@@ -220,6 +227,8 @@ size_t m2l_f64_part_doubles(int p);           // class-group sums of one tile
 void m2l_pass_tc(Workspace &ws);              // M2L into L (tensor cores, mixed)
 bool m2l_tc_supported(int p);
 size_t m2l_tc_image_floats(int p);
+unsigned m2l_tc_tiles(const Workspace &ws);   // bound of the tiles of ws.c_cap cells
+size_t m2l_tc_part_floats(int p, unsigned tiles, unsigned ctas);
 int m2l_tc_row_floats(int p);
 const char *m2l_tc_encode(Workspace &ws);     // (re)build tmap_ms; nullptr or an error message
 void downward_pass(Workspace &ws);            // L2L + L2P into far
@@ -250,6 +259,18 @@ int generate_clustered(Workspace &ws, unsigned n, uint64_t seed, int clusters, d
                        double *params);
 void direct_sum(Workspace &ws, const double *x_orig, const long long *targets, unsigned nt, double *out_soa,
                 double *part, unsigned nsplit);  // part: [nsplit][3][nt] scratch
+
+#ifdef __CUDACC__
+// Every kernel that may run beside the near field asks for the same split of an
+// SM's memory as P2P does (full shared memory): an SM changes its split only when
+// it is idle, so a far-field kernel with another preference waited until the
+// persistent P2P blocks were done (a forest's operator kernel started 20 ms late
+// and the far field ran after the near field instead of beside it).
+template <typename F>
+inline void full_shared(F *kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+#endif
 
 // timing helpers
 void timer_begin(Workspace &ws, int cls);
