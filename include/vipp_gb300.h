@@ -288,7 +288,7 @@ typedef struct gb_tuning {
     int p2p_blocks;      /* P2P blocks per SM when the near field runs alone, 1..16 (default 8) */
     int p2p_blocks_conc; /* P2P blocks per SM launched beside the far field, 0..16 (default 8) */
     int p2p_slice;       /* near-field sources per P2P work item, 1024..65536 (default 8192);
-                            small systems take shorter ones (n / 8, FP64 n / 32) */
+                            small systems take shorter ones (n / 32) */
     int m2l_ctas_pct;    /* tensor-core M2L CTAs, percent of the SMs, 10..100 (default 100) */
     int serial;          /* 1: the near field after the far field on one stream (default 0) */
     int leaf_s;          /* GB_MODE_ACCURATE: leaf parameter used instead of the config's s

@@ -435,11 +435,30 @@ int check_device_errors(gb_ctx *ctx, unsigned *need) {
 void evaluate(gb_ctx *ctx, bool to_acc = true) {
     gb::Workspace &ws = ctx->ws;
     g_timer_ctx = ctx;
+    gb::tree_box(ws);
+    const bool fork = !ws.serial && !ws.timing;
+    // The operators follow from the root box alone, so a single tree's are built
+    // beside the tree (54 of the far field's 430 us at 100,003 particles). A forest's
+    // take as long as its tree and write gigabytes of images: beside the tree they
+    // delay the near field, which bounds the step (512 systems 134.7 -> 141 ms), so
+    // they run at the start of the far field.
+    const bool fork_ops = fork && !ws.forest();
+    auto operators = [&]() {
+        gb::build_operators(ws);
+        if (ws.m2l_tensor) gb::m2l_tc_images(ws);
+    };
+    if (fork_ops) {
+        cudaEventRecord(ws.ev_box, ws.st);
+        cudaStreamWaitEvent(ws.st4, ws.ev_box, 0);
+        std::swap(ws.st, ws.st4);
+        operators();
+        std::swap(ws.st, ws.st4);
+        cudaEventRecord(ws.ev_ops, ws.st4);
+    }
     gb::build_tree(ws);
     if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : ws.mixed ? gb::kM2LTileCC : gb::kM2LTileF64);
     // Near field on the second stream, unless serial or timed: class timers
     // measure each class alone on one stream.
-    const bool fork = !ws.serial && !ws.timing;
     // Beside the far field, no more P2P blocks per SM than its tensor-core M2L leaves
     // registers for (m2l_tc.cu): with more, the M2L's CTAs only
     // start when the near field is done. Three against eight (then one after the
@@ -470,8 +489,10 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
         std::swap(ws.st, ws.st3);
         cudaEventRecord(ws.ev_join3, ws.st3);
     }
-    gb::build_operators(ws);
-    gb::upward_pass(ws);
+    if (!fork_ops) operators();
+    gb::p2m_pass(ws);
+    if (fork_ops) cudaStreamWaitEvent(ws.st, ws.ev_ops, 0);
+    gb::m2m_pass(ws);
     if (ws.m2l_tensor)
         gb::m2l_pass_tc(ws);
     else
@@ -723,6 +744,9 @@ int gb_create(const gb_config *cfg, gb_ctx **out) {
     if ((e = cudaEventCreateWithFlags(&ws.ev_fork, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
     if ((e = cudaEventCreateWithFlags(&ws.ev_join, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
     if ((e = cudaStreamCreateWithFlags(&ws.st3, cudaStreamNonBlocking)) != cudaSuccess) return fail("stream", e);
+    if ((e = cudaStreamCreateWithFlags(&ws.st4, cudaStreamNonBlocking)) != cudaSuccess) return fail("stream", e);
+    if ((e = cudaEventCreateWithFlags(&ws.ev_box, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
+    if ((e = cudaEventCreateWithFlags(&ws.ev_ops, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
     if ((e = cudaEventCreateWithFlags(&ws.ev_fork3, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
     if ((e = cudaEventCreateWithFlags(&ws.ev_join3, cudaEventDisableTiming)) != cudaSuccess) return fail("event", e);
     if ((e = gb::upload_tables()) != cudaSuccess) return fail("tables", e);
@@ -768,6 +792,9 @@ void gb_destroy(gb_ctx *ctx) {
     if (ctx->step_exec) cudaGraphExecDestroy(ctx->step_exec);
     if (ws.ev_fork) cudaEventDestroy(ws.ev_fork);
     if (ws.ev_join) cudaEventDestroy(ws.ev_join);
+    if (ws.ev_box) cudaEventDestroy(ws.ev_box);
+    if (ws.ev_ops) cudaEventDestroy(ws.ev_ops);
+    if (ws.st4) cudaStreamDestroy(ws.st4);
     if (ws.ev_fork3) cudaEventDestroy(ws.ev_fork3);
     if (ws.ev_join3) cudaEventDestroy(ws.ev_join3);
     if (ws.st3) cudaStreamDestroy(ws.st3);

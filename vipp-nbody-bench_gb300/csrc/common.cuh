@@ -116,26 +116,36 @@ GB_HD void chunk_at(int n, int q, int &off, int &len) {
 // are added in slice order afterwards. This bounds the longest work item.
 constexpr int kSliceSources = 8192;  // default; the tuning may pick another length
 constexpr int kMaxSlices = 4095;
-// Small systems take shorter slices: their few leaves would leave most warps of
-// the GPU without an item (16,384 particles: about 900 items of 3,700 sources for
-// 3,648 resident warps). FP64 pairs hold the FP64 pipe for 384 cycles each, so
-// those slices are n / 32 sources, at least 128 (16,384 particles: near field
-// 3.68 -> 0.88 ms per evaluation, 4.65 without slices below 8,192); FP32 slices
-// are n / 8, at least 512 (3,001 particles 0.12 -> 0.025 ms), since shorter ones
-// cost a batch of many systems, whose items fill the GPU anyway, more than they
-// give (512 systems: 88.2 ms without, 91.4 with n / 32). The length follows from
-// the system's own particle count, so a forest's system sums its sources in the
-// same order as in a context of its own.
-GB_HD unsigned slice_length(unsigned n, unsigned slice, bool fp32) {
-    const unsigned lo = fp32 ? 512u : 128u, s = (fp32 ? n / 8 : n / 32) / 32 * 32;
-    const unsigned q = s < lo ? lo : s;
+// Small systems take shorter slices, n / 32 sources and at least 256: their few
+// leaves would leave most warps of the GPU without an item (16,384 particles:
+// about 900 items of 3,700 sources for 3,648 resident warps; near field in FP64
+// 3.68 -> 0.88 ms per evaluation). The length follows from the system's own
+// particle count, so a forest's system sums its sources in the same order as in
+// a context of its own; the items of a forest take as many consecutive slices as
+// its total particle count asks for (slices_per_item), since its many systems
+// fill the GPU anyway (512 systems: 88.2 ms per step, 91.4 with an item per slice).
+GB_HD unsigned slice_length(unsigned n, unsigned slice) {
+    const unsigned q = n / 32 < 256 ? 256 : n / 32;
     return q < slice ? q : slice;
 }
-GB_HD int slice_count(unsigned long long srcs, unsigned slice = kSliceSources) {
-    const unsigned long long s = (srcs + slice - 1) / slice;
-    return s < 1 ? 1 : (s > kMaxSlices ? kMaxSlices : static_cast<int>(s));
+// A leaf's slice length: its sources in equal slices, a multiple of the 32-source
+// batches (only a list's last batch is partial), at most kMaxSlices of them.
+GB_HD unsigned leaf_slice(unsigned long long srcs, unsigned n_sys, unsigned slice) {
+    const unsigned long long q = slice_length(n_sys, slice);
+    unsigned long long ns = (srcs + q - 1) / q;
+    ns = ns < 1 ? 1 : (ns > kMaxSlices ? kMaxSlices : ns);
+    const unsigned long long per = ((srcs + ns - 1) / ns + 31) / 32 * 32;
+    return per < 32 ? 32u : static_cast<unsigned>(per);
 }
-// Work-item field z: targets (6 bits), slice index (12 bits), slices (12 bits).
+GB_HD int slice_count(unsigned long long srcs, unsigned slice) {
+    const unsigned long long s = (srcs + slice - 1) / slice;
+    return s < 1 ? 1 : static_cast<int>(s);
+}
+GB_HD int slices_per_item(unsigned n_total, unsigned slice, unsigned leaf_len) {
+    const unsigned k = slice_length(n_total, slice) / leaf_len;
+    return k < 1 ? 1 : static_cast<int>(k);
+}
+// Work-item field z: targets (6 bits), first slice (12 bits), the leaf's slices (12 bits).
 GB_HD int item_pack(int nt, int s, int ns) { return nt | (s << 6) | (ns << 18); }
 GB_HD int item_nt(int z) { return z & 63; }
 GB_HD int item_slice(int z) { return (z >> 6) & 4095; }

@@ -577,24 +577,56 @@ __device__ __forceinline__ void tile_clear(T *sm) {
     for (int i = threadIdx.x; i < (kTile + C::KO) * C::KS; i += blockDim.x) sm[i] = T(0);
 }
 
-// Op tile <- operator oi (global, output-major K x K).
+// Both loads read kLoadBatch values into registers before storing any: a value at
+// a time, the 20 to 60 dependent trips to L2 made a level of one tile cost ~24 us
+// at p = 8 (M2M and L2L; 11 us with the batches).
+constexpr int kLoadBatch = 8;
+
+// Op tile <- operator oi (global, output-major K x K); 256 threads.
 template <int P, typename T>
 __device__ __forceinline__ void tile_load_op(T *Op, const T *__restrict__ ops, int oi) {
     using C = TileCfg<P, T>;
     const T *op = ops + static_cast<size_t>(oi) * C::K * C::K;
-    for (int i = threadIdx.x; i < C::K * C::K; i += blockDim.x) Op[(i / C::K) * C::KS + i % C::K] = op[i];
-}
-
-// A row t <- expansion of cell src[t] (zero when src[t] < 0).
-template <int P, typename T>
-__device__ __forceinline__ void tile_gather(T *A, const int *srcs, const T *__restrict__ X) {
-    using C = TileCfg<P, T>;
-    for (int i = threadIdx.x; i < kTile * C::K; i += blockDim.x) {
-        const int t = i / C::K, ci = i % C::K;
-        const int s = srcs[t];
-        A[t * C::KS + ci] = s >= 0 ? X[static_cast<size_t>(s) * C::K + ci] : T(0);
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < C::K * C::K; i0 += 256 * kLoadBatch) {
+        T v[kLoadBatch];
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) v[u] = i0 + 256 * u < C::K * C::K ? __ldg(op + i0 + 256 * u) : T(0);
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) {
+            const int i = i0 + 256 * u;
+            if (i < C::K * C::K) Op[(i / C::K) * C::KS + i % C::K] = v[u];
+        }
     }
 }
+
+// A row t <- expansion of cell src[t] (zero when src[t] < 0), t < rows; 256 threads.
+template <int P, typename T>
+__device__ __forceinline__ void tile_gather(T *A, const int *srcs, const T *X, int rows = kTile) {
+    using C = TileCfg<P, T>;
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < rows * C::K; i0 += 256 * kLoadBatch) {
+        T v[kLoadBatch];
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) {
+            const int i = i0 + 256 * u, t = i / C::K;
+            const int s = i < rows * C::K ? srcs[t] : -1;
+            v[u] = s >= 0 ? X[static_cast<size_t>(s) * C::K + (i - t * C::K)] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) {
+            const int i = i0 + 256 * u, t = i / C::K;
+            if (i < rows * C::K) A[t * C::KS + (i - t * C::K)] = v[u];
+        }
+    }
+}
+
+// Rows of an M2M or L2L tile: 64, or 16 while a level's tiles of 16 still run
+// side by side (`slots` of them): a small level then spreads over four times the
+// SMs, and a tile's gather and product take a quarter of the time. The rows'
+// arithmetic is the same either way.
+constexpr int kTileSmall = 16;
+__device__ __forceinline__ int level_rows(int cnt, int slots) { return (cnt + kTileSmall - 1) / kTileSmall <= slots ? kTileSmall : kTile; }
 
 // --------------------------------------------------------------------- M2M
 // One block per non-leaf cell of level L (>= 2): M~ = sum_o M2M_o M~_child(o).
@@ -698,16 +730,17 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, sizeof(T) == 4 
     const int e0 = info->split_start[L], cnt = info->split_count[L];
     // a forest's tiles: one system each, with that system's operator
     const int et0 = etile ? info->etile_start[L] : 0;
-    const int tiles = etile ? info->etile_end[L] - et0 : (cnt + kTile - 1) / kTile;
+    const int nclusters = static_cast<int>(gridDim.x) / 8;
+    const int R = etile ? kTile : level_rows(cnt, nclusters);
+    const int tiles = etile ? info->etile_end[L] - et0 : (cnt + R - 1) / R;
     // uniform over each cluster (it shares blockIdx.x / 8): a cluster without a
     // tile reaches no cluster barrier and skips loading its operator
     if (static_cast<int>(blockIdx.x) / 8 >= tiles) return;
     tile_clear<P, T>(A);
     __syncthreads();  // Op is cleared before any thread loads its part of the operator
     int loaded = -1;  // system whose operator is in Op
-    const int nclusters = static_cast<int>(gridDim.x) / 8;
     for (int w = static_cast<int>(blockIdx.x) / 8; w < tiles; w += nclusters) {  // same w in all 8 CTAs
-        int first = e0 + w * kTile, count = cnt - w * kTile, sys = 0;
+        int first = e0 + w * R, count = min(cnt - w * R, R), sys = 0;
         if (etile) {
             const int2 et = etile[et0 + w];
             first = et.x, count = et.y, sys = c_sys[split_cell[first]];
@@ -721,7 +754,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, sizeof(T) == 4 
             srcs[tid] = par[tid] >= 0 ? c_child[par[tid]] + o : -1;
         }
         __syncthreads();
-        tile_gather<P, T>(A, srcs, M);
+        tile_gather<P, T>(A, srcs, M, R);
         __syncthreads();
         T acc[4][C::NJ];
 #pragma unroll
@@ -730,16 +763,17 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, sizeof(T) == 4 
             for (int j = 0; j < C::NJ; ++j) acc[a][j] = 0;
         if (ty * 4 < count) tile_gemm<P, T>(A, Op, acc, ty, tx);  // rows past the tile's parents are not stored
         __syncthreads();
+        if (ty * 4 < R)
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int j = 0; j < C::NJ; ++j) {
-                const int r = tx + 16 * j;
-                if (r < C::K) A[(ty * 4 + a) * C::KS + r] = acc[a][j];
-            }
+                for (int j = 0; j < C::NJ; ++j) {
+                    const int r = tx + 16 * j;
+                    if (r < C::K) A[(ty * 4 + a) * C::KS + r] = acc[a][j];
+                }
         cluster.sync();  // all eight partial tiles written
-        for (int i = tid; i < 8 * C::K; i += blockDim.x) {
-            const int row = 8 * o + i / C::K, r = i % C::K;
+        for (int i = tid; i < R / 8 * C::K; i += blockDim.x) {
+            const int row = R / 8 * o + i / C::K, r = i % C::K;
             const int pc = par[row];
             if (pc < 0) continue;
             T sum = 0;
@@ -765,12 +799,13 @@ __global__ void __launch_bounds__(256, GB_FAR_MIN_BLOCKS) k_l2l(int Lp, const Tr
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     const int e0 = info->split_start[Lp], cnt = info->split_count[Lp];
     const int et0 = etile ? info->etile_start[Lp] : 0;
-    const int tiles = etile ? info->etile_end[Lp] - et0 : (cnt + kTile - 1) / kTile;
+    const int R = etile ? kTile : level_rows(cnt, static_cast<int>(gridDim.x) / 8);
+    const int tiles = etile ? info->etile_end[Lp] - et0 : (cnt + R - 1) / R;
     if (static_cast<int>(blockIdx.x) >= 8 * tiles) return;  // no (tile, octant) for this block
     tile_clear<P, T>(A);
     for (int w = blockIdx.x; w < 8 * tiles; w += gridDim.x) {
         const int o = w % 8, tile = w / 8;
-        int first = e0 + tile * kTile, count = cnt - tile * kTile, sys = 0;
+        int first = e0 + tile * R, count = min(cnt - tile * R, R), sys = 0;
         if (etile) {
             const int2 et = etile[et0 + tile];
             first = et.x, count = et.y, sys = c_sys[split_cell[first]];
@@ -779,7 +814,7 @@ __global__ void __launch_bounds__(256, GB_FAR_MIN_BLOCKS) k_l2l(int Lp, const Tr
         if (tid < kTile) par[tid] = tid < count ? split_cell[first + tid] : -1;
         __syncthreads();
         tile_load_op<P, T>(Op, ops_all + static_cast<size_t>(sys) * kNumOps * C::K * C::K, kOpL2L + o);
-        tile_gather<P, T>(A, par, Lx);
+        tile_gather<P, T>(A, par, Lx, R);
         __syncthreads();
         T acc[4][C::NJ];
 #pragma unroll
@@ -787,16 +822,23 @@ __global__ void __launch_bounds__(256, GB_FAR_MIN_BLOCKS) k_l2l(int Lp, const Tr
 #pragma unroll
             for (int j = 0; j < C::NJ; ++j) acc[a][j] = 0;
         if (ty * 4 < count) tile_gemm<P, T>(A, Op, acc, ty, tx);
+        // all loads of the children's expansions before the first store (one by one,
+        // the 24 round trips cost ~8 us)
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int pc = par[ty * 4 + a];
-            if (pc < 0) continue;
-            const size_t c = static_cast<size_t>(c_child[pc] + o);
+            T *out = Lx + static_cast<size_t>(pc >= 0 ? c_child[pc] + o : 0) * C::K;
 #pragma unroll
-            for (int j = 0; j < C::NJ; ++j) {
-                const int r = tx + 16 * j;
-                if (r < C::K) Lx[c * C::K + r] += acc[a][j];
-            }
+            for (int j = 0; j < C::NJ; ++j)
+                if (pc >= 0 && tx + 16 * j < C::K) acc[a][j] = out[tx + 16 * j] + acc[a][j];
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int pc = par[ty * 4 + a];
+            T *out = Lx + static_cast<size_t>(pc >= 0 ? c_child[pc] + o : 0) * C::K;
+#pragma unroll
+            for (int j = 0; j < C::NJ; ++j)
+                if (pc >= 0 && tx + 16 * j < C::K) out[tx + 16 * j] = acc[a][j];
         }
     }
 }
@@ -976,7 +1018,7 @@ void launch_m2m_levels(Workspace &ws) {
     const size_t smem = TileCfg<P, T>::smem;
     cudaFuncSetAttribute(k_m2m<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     full_shared(k_m2m<P, T>);
-    const unsigned gs = 8 * capped_grid(static_cast<unsigned>(ws.num_sms) / 8 * 2, ceil_div(ws.s_cap, kTile));  // clusters of 8 CTAs
+    const unsigned gs = 8 * capped_grid(static_cast<unsigned>(ws.num_sms) / 8 * 2, ceil_div(ws.s_cap, kTileSmall));  // clusters of 8 CTAs
     // no cell is deeper than the key levels the sort ordered (tree.cu), so
     // parents lie at levels < ws.sort_levels
     for (int L = ws.sort_levels - 1; L >= 2; --L) {
@@ -991,7 +1033,7 @@ void launch_l2l_levels(Workspace &ws) {
     const size_t smem = TileCfg<P, T>::smem;
     cudaFuncSetAttribute(k_l2l<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     full_shared(k_l2l<P, T>);
-    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2, 8 * ceil_div(ws.s_cap, kTile));
+    const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2, 8 * ceil_div(ws.s_cap, kTileSmall));
     for (int Lp = 2; Lp <= ws.sort_levels - 1; ++Lp) {
         k_l2l<P, T><<<gs, 256, smem, ws.st>>>(Lp, ws.info, ws.split_cell, ws.c_child, ops_of<P, T>(ws),
                                               ws.forest() ? ws.etile : nullptr, ws.c_sys, static_cast<T *>(ws.Lexp));
@@ -1050,8 +1092,10 @@ void build_operators(Workspace &ws) {
         // M2L offsets: FP32 operators, kSysPerBlock systems per block; then M2M and L2L
         // few systems: a thread per order (latency); many: a thread per operator (FP64 work)
         const int cols = nsys < 16 ? 2 * ws.p + 1 : 1;
-        full_shared(k_zf_tables);
-        full_shared(k_build_ops_f);
+        if (ws.forest()) {  // beside the near field (a single tree's: beside the tree build)
+            full_shared(k_zf_tables);
+            full_shared(k_build_ops_f);
+        }
         k_zf_tables<<<static_cast<unsigned>(ceil_div(static_cast<size_t>(nsys) * kNumOps * cols, 128)), 128, 0, ws.st>>>(
             ws.info, nsys, ws.p, cols, ws.zf);
         const size_t smem_f = kSysPerBlock * sizeof(float) * ny;
@@ -1059,7 +1103,7 @@ void build_operators(Workspace &ws) {
             nsys, ws.p, static_cast<const M2LEnt *>(ws.m2l_tab), ws.zf, ws.ops_f);
         ws.launches += 1;
     } else {
-        full_shared(k_build_ops);
+        if (ws.forest()) full_shared(k_build_ops);
         k_build_ops<<<dim3(kNumOps, nsys), 256, smem, ws.st>>>(ws.info, ws.p, static_cast<const M2LEnt *>(ws.m2l_tab), ws.ops_d,
                                                               ws.ops_f, false, 0);
     }
@@ -1067,16 +1111,22 @@ void build_operators(Workspace &ws) {
     timer_end(ws, kTOps);
 }
 
-void upward_pass(Workspace &ws) {
+void p2m_pass(Workspace &ws) {
     timer_begin(ws, kTUp);
-    if (ws.mixed) {
+    if (ws.mixed)
         dispatch_p<float>(ws, 0);
-        dispatch_p<float>(ws, 3);
-    } else {
+    else
         dispatch_p<double>(ws, 0);
-        dispatch_p<double>(ws, 3);
-    }
     ws.launches += 1;
+    timer_end(ws, kTUp);
+}
+
+void m2m_pass(Workspace &ws) {
+    timer_begin(ws, kTUp);
+    if (ws.mixed)
+        dispatch_p<float>(ws, 3);
+    else
+        dispatch_p<double>(ws, 3);
     timer_end(ws, kTUp);
 }
 

@@ -87,7 +87,7 @@ constexpr int kParts = (kSlotsPerTile + kPartSlots - 1) / kPartSlots;
 constexpr int kPartGroups = kPartSlots / kGroup;
 static_assert(kPartSlots % kGroup == 0, "parts of whole groups");
 constexpr int kSmemMax = 232448;    // opt-in shared memory per block
-constexpr int kSmemBeside = kSmemMax - 4 * 4352;  // what four P2P blocks leave of an SM's
+constexpr int kSmemBeside = kSmemMax - 3 * 5760;  // what three P2P blocks leave of an SM's
 
 template <int P, bool BF>
 struct TcCfg {
@@ -744,17 +744,23 @@ __global__ void k_build_bimg(const float *__restrict__ ops_all, unsigned char *_
 }
 
 template <int P, bool BF>
-void launch(Workspace &ws) {
+void launch_images(Workspace &ws) {
     using C = TcCfg<P, BF>;
-    const bool forest = ws.forest();
     const int op_smem = static_cast<int>(sizeof(float) * C::K * C::K);
     if (op_smem > 48 * 1024)
         cudaFuncSetAttribute(k_build_bimg<P, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, op_smem);
-    full_shared(k_build_bimg<P, BF>);
+    if (ws.forest()) full_shared(k_build_bimg<P, BF>);
+    k_build_bimg<P, BF><<<dim3(kNumOffsets, ws.forest() ? ws.nsys : 1), 256, op_smem, ws.st>>>(
+        ws.ops_f, reinterpret_cast<unsigned char *>(ws.bimg));
+    ws.launches += 1;
+}
+
+template <int P, bool BF>
+void launch(Workspace &ws) {
+    using C = TcCfg<P, BF>;
+    const bool forest = ws.forest();
     full_shared(k_split_m<P, BF>);
     full_shared(k_m2l_tc<P, BF>);
-    k_build_bimg<P, BF><<<dim3(kNumOffsets, forest ? ws.nsys : 1), 256, op_smem, ws.st>>>(ws.ops_f,
-                                                                                 reinterpret_cast<unsigned char *>(ws.bimg));
     k_split_m<P, BF><<<4 * ws.num_sms, 256, 0, ws.st>>>(ws.info, static_cast<const float *>(ws.Mexp), ws.ms_tc,
                                                         static_cast<int>(ws.ms_rows), ws.m2l_tc_pcnt,
                                                         static_cast<int>(ws.m2l_tc_tiles));
@@ -766,15 +772,30 @@ void launch(Workspace &ws) {
                                                       forest ? ws.otile : nullptr, ws.oct_list,
                                                       static_cast<int>(ws.ms_rows), static_cast<float *>(ws.Lexp), ws.info,
                                                       ws.m2l_tc_part, ws.m2l_tc_pcnt, static_cast<int>(ws.m2l_tc_tiles));
-    ws.launches += 3;
+    ws.launches += 2;
 }
 
 template <int P>
-void launch_kind(Workspace &ws) {
-    if (ws.m2l_bf16)
-        launch<P, true>(ws);
+void launch_kind(Workspace &ws, bool images) {
+    if (images)
+        ws.m2l_bf16 ? launch_images<P, true>(ws) : launch_images<P, false>(ws);
     else
-        launch<P, false>(ws);
+        ws.m2l_bf16 ? launch<P, true>(ws) : launch<P, false>(ws);
+}
+
+void launch_p(Workspace &ws, bool images) {
+    switch (ws.p) {
+        case 2: launch_kind<2>(ws, images); break;
+        case 3: launch_kind<3>(ws, images); break;
+        case 4: launch_kind<4>(ws, images); break;
+        case 5: launch_kind<5>(ws, images); break;
+        case 6: launch_kind<6>(ws, images); break;
+        case 7: launch_kind<7>(ws, images); break;
+        case 8: launch_kind<8>(ws, images); break;
+        case 9: launch_kind<9>(ws, images); break;
+        case 10: launch_kind<10>(ws, images); break;
+        default: break;
+    }
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -835,20 +856,15 @@ const char *m2l_tc_encode(Workspace &ws) {
     return nullptr;
 }
 
+void m2l_tc_images(Workspace &ws) {
+    timer_begin(ws, kTM2L);
+    launch_p(ws, true);
+    timer_end(ws, kTM2L);
+}
+
 void m2l_pass_tc(Workspace &ws) {
     timer_begin(ws, kTM2L);
-    switch (ws.p) {
-        case 2: launch_kind<2>(ws); break;
-        case 3: launch_kind<3>(ws); break;
-        case 4: launch_kind<4>(ws); break;
-        case 5: launch_kind<5>(ws); break;
-        case 6: launch_kind<6>(ws); break;
-        case 7: launch_kind<7>(ws); break;
-        case 8: launch_kind<8>(ws); break;
-        case 9: launch_kind<9>(ws); break;
-        case 10: launch_kind<10>(ws); break;
-        default: break;
-    }
+    launch_p(ws, false);
     timer_end(ws, kTM2L);
 }
 

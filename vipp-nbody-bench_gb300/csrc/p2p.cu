@@ -93,20 +93,16 @@ struct BatchCursor {
     }
 };
 
-// Work item -> (leaf, first target, targets, slice, slices, partial slot,
-// source slice [v0, v0 + len)).
+// Work item -> (leaf, first target, targets, slices [sl, se) of ns, slot of the
+// first slice's partial sums). An item with all of its leaf's slices adds their
+// sums in slice order itself; else k_p2p_combine does.
 struct Item {
-    int li, t0, nt, sl, ns, pslot;
-    unsigned v0, len;
+    int li, t0, nt, sl, se, ns, pslot;
     __device__ __forceinline__ explicit Item(const int4 w)
         : li(w.x), t0(w.y), nt(item_nt(w.z)), sl(item_slice(w.z)), ns(item_nslices(w.z)), pslot(w.w) {}
-    __device__ __forceinline__ void slice(unsigned S) {
-        const unsigned per = (S + ns - 1) / ns;
-        v0 = min(S, sl * per);
-        len = min(per, S - v0);
-    }
+    __device__ __forceinline__ void of_leaf(int spi) { se = min(ns, sl + spi); }
+    __device__ __forceinline__ bool whole() const { return sl == 0 && se == ns; }
 };
-
 // A source pair (j, j') against a target on paired FP32 instructions (.f32x2);
 // each component rounds exactly like the scalar operation.
 template <bool kNewton, bool kSoft>
@@ -138,14 +134,16 @@ constexpr float kNowhere = 1e18f;
 // ms, 4.92 before; 1M unit cube 0.475 -> 0.465; 1M at p = 10 2.06 -> 1.96). A
 // 64-register build (8 blocks) spills 24 bytes and measured 1-5% slower on every
 // workload; a 96-register build kept the cluster M2M from starting beside P2P.
-template <bool kNewton, bool kSoft>
+// kMulti: items of several consecutive slices (a forest's); a single tree's items are
+// one slice each, and the bookkeeping between slices costs the kernel 1.7%.
+template <bool kNewton, bool kSoft, bool kMulti>
 __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__restrict__ chunks, const unsigned *counts,
                                                             unsigned *queue, const LeafRec *__restrict__ recs,
                                                             const uint2 *__restrict__ ranges, const float4 *__restrict__ ph,
                                                             const float4 *__restrict__ pl, float *__restrict__ part, float Gm,
                                                             float eps2, float *__restrict__ nearv, unsigned n) {
     __shared__ __align__(16) float src[kP2PWarps][3][32];  // the staged batch, leaf-relative
-    __shared__ float red[kP2PWarps][3][32];
+    __shared__ float red[kP2PWarps][3][32], sum[kMulti ? kP2PWarps : 1][3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
     unsigned ci = 0;
@@ -155,7 +153,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
         if (ci >= nch) break;
         Item it(chunks[ci]);
         const LeafRec rec = recs[it.li];
-        it.slice(rec.src_total);
+        it.of_leaf(rec.spi);
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
@@ -172,15 +170,32 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
             txy = __fadd2_rn(__fadd2_rn(make_float2(h.x, h.y), chxy), __fadd2_rn(make_float2(l.x, l.y), clxy));
             tz = (h.z + chz) + (l.z + clz);
         }
+        const float2 ntx = make_float2(-txy.x, -txy.x), nty = make_float2(-txy.y, -txy.y), ntz = make_float2(-tz, -tz);
+        const float2 e2 = make_float2(eps2, eps2);
+        // Consecutive slices share one stream of batches (a batch ends with its slice);
+        // a slice's sum goes to the item's sums in shared memory, or to its slot.
+        if (kMulti) sum[w][0][lane] = 0.f, sum[w][1][lane] = 0.f, sum[w][2][lane] = 0.f;
         float sx = 0, sy = 0, sz = 0, kx = 0, ky = 0, kz = 0;  // Kahan sums and compensations
+        auto slice_sum = [&]() {  // of the lane groups, in group 0
+            sx -= kx, sy -= ky, sz -= kz;
+            if (g > 1) {
+                red[w][0][lane] = sx, red[w][1][lane] = sy, red[w][2][lane] = sz;
+                __syncwarp();
+                if (grp == 0)
+                    for (int q = 1; q < g; ++q)
+                        sx += red[w][0][t + q * nt], sy += red[w][1][t + q * nt], sz += red[w][2][t + q * nt];
+                __syncwarp();
+            }
+        };
+        int sl = it.sl;
+        const unsigned v0 = min(rec.src_total, static_cast<unsigned>(sl) * rec.slice);
+        unsigned left = rec.src_total - v0;  // sources from this slice on
         BatchCursor cur;
-        cur.start(ranges + rec.rng_off, rec.rng_len, it.v0, it.len, static_cast<unsigned>(lane));
+        cur.start(ranges + rec.rng_off, rec.rng_len, v0, min(rec.slice, left), static_cast<unsigned>(lane));
         float4 h = make_float4(0, 0, 0, 0), l = h;
         unsigned sidx;
         unsigned cnt = cur.next(static_cast<unsigned>(lane), sidx);
         if (static_cast<unsigned>(lane) < cnt) h = ph[sidx], l = pl[sidx];
-        const float2 ntx = make_float2(-txy.x, -txy.x), nty = make_float2(-txy.y, -txy.y), ntz = make_float2(-tz, -tz);
-        const float2 e2 = make_float2(eps2, eps2);
         bool taken = false;
         while (cnt) {
             const bool on = static_cast<unsigned>(lane) < cnt;
@@ -189,12 +204,16 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
             src[w][1][lane] = xy.y;
             src[w][2][lane] = (h.z + chz) + (l.z + clz);
             __syncwarp();
-            cnt = cur.next(static_cast<unsigned>(lane), sidx);  // prefetch the next batch while this one is computed
-            if (static_cast<unsigned>(lane) < cnt) h = ph[sidx], l = pl[sidx];
-            if (cur.rem == 0 && !taken) {  // the slice's last batch is on its way: take the next item
+            const bool ends = cur.rem == 0;  // the staged batch is its slice's last
+            if (kMulti && ends && ++sl < it.se) {
+                left -= rec.slice;
+                cur.rem = min(rec.slice, left);
+            } else if (ends && !taken) {  // nothing more to fetch: take the next item
                 taken = true;
                 if (lane == 0) ci = atomicAdd(queue, 1u);
             }
+            cnt = cur.next(static_cast<unsigned>(lane), sidx);  // prefetch the next batch while this one is computed
+            if (static_cast<unsigned>(lane) < cnt) h = ph[sidx], l = pl[sidx];
             float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
             if (g == 1) {
 #pragma unroll
@@ -221,22 +240,28 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
             ky = (tt - sy) - y, sy = tt;
             y = (az.x + az.y) - kz, tt = sz + y;
             kz = (tt - sz) - y, sz = tt;
+            if (kMulti && ends) {
+                slice_sum();
+                if (it.whole()) {
+                    sum[w][0][lane] += sx, sum[w][1][lane] += sy, sum[w][2][lane] += sz;
+                } else if (grp == 0) {  // sl is already the next slice
+                    float *o = part + static_cast<size_t>(it.pslot + sl - 1 - it.sl) * 96;
+                    o[t] = sx, o[32 + t] = sy, o[64 + t] = sz;
+                }
+                sx = sy = sz = kx = ky = kz = 0;
+            }
         }
-        if (!taken && lane == 0) ci = atomicAdd(queue, 1u);  // an empty slice
-        sx -= kx, sy -= ky, sz -= kz;
-        if (g > 1) {
-            red[w][0][lane] = sx, red[w][1][lane] = sy, red[w][2][lane] = sz;
-            __syncwarp();
-            if (grp == 0)
-                for (int q = 1; q < g; ++q) sx += red[w][0][t + q * nt], sy += red[w][1][t + q * nt], sz += red[w][2][t + q * nt];
-            __syncwarp();
-        }
+        if (!taken && lane == 0) ci = atomicAdd(queue, 1u);  // no sources
+        if (kMulti)
+            sx = sum[w][0][lane], sy = sum[w][1][lane], sz = sum[w][2][lane];
+        else
+            slice_sum();
         if (grp == 0) {
-            if (it.ns == 1) {
+            if (it.whole()) {
                 nearv[i] = Gm * sx;
                 nearv[n + i] = Gm * sy;
                 nearv[2 * static_cast<size_t>(n) + i] = Gm * sz;
-            } else {
+            } else if (!kMulti) {
                 float *o = part + static_cast<size_t>(it.pslot) * 96;
                 o[t] = sx, o[32 + t] = sy, o[64 + t] = sz;
             }
@@ -245,13 +270,13 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
 }
 
 template <bool kSoft>
-__global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restrict__ chunks, const unsigned *counts,
+__global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__restrict__ chunks, const unsigned *counts,
                                                             unsigned *queue, const LeafRec *__restrict__ recs,
                                                             const uint2 *__restrict__ ranges, const double *__restrict__ xs,
                                                             double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ nearv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
-    __shared__ double red[kP2PWarps][3][32];
+    __shared__ double red[kP2PWarps][3][32], sum[kP2PWarps][3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
     while (true) {
@@ -260,8 +285,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
         ci = __shfl_sync(0xffffffffu, ci, 0);
         if (ci >= nch) break;
         Item it(chunks[ci]);
-        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total
-        it.slice(rec.z);
+        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total, spi
+        const unsigned slice = recs[it.li].slice;
+        it.of_leaf(static_cast<int>(rec.w));
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
@@ -269,64 +295,70 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_f64(const int4 *__restri
         const bool tact = grp < g;
         const int i = it.t0 + t;
         const double tx = tact ? xs[i] : 0.0, ty = tact ? xs[n + i] : 0.0, tz = tact ? xs[2 * static_cast<size_t>(n) + i] : 0.0;
-        double ax = 0, ay = 0, az = 0;
-        BatchCursor cur;
-        cur.start(ranges + rec.x, rec.y, it.v0, it.len, static_cast<unsigned>(lane));
-        unsigned j;
-        for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
-            if (static_cast<unsigned>(lane) < cnt) {
-                src[w][0][lane] = xs[j];
-                src[w][1][lane] = xs[n + j];
-                src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
-            }
-            __syncwarp();
-            if (tact)
-#pragma unroll 2
-                for (unsigned k = grp; k < cnt; k += g) {
-                    const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
-                    double f;
-                    if (!rinv3(dx, dy, dz, soft, f)) {
-                        const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                        double ri = rsqrt(r2);
-                        if (!kSoft) ri = r2 > 0.0 ? ri : 0.0;
-                        f = ri * ri * ri;
-                    }
-                    ax += f * dx;
-                    ay += f * dy;
-                    az += f * dz;
+        sum[w][0][lane] = 0, sum[w][1][lane] = 0, sum[w][2][lane] = 0;  // the finished slices' sums
+        for (int sl = it.sl; sl < it.se; ++sl) {
+            unsigned v0, len;
+            v0 = min(rec.z, static_cast<unsigned>(sl) * slice), len = min(slice, rec.z - v0);
+            double ax = 0, ay = 0, az = 0;
+            BatchCursor cur;
+            cur.start(ranges + rec.x, rec.y, v0, len, static_cast<unsigned>(lane));
+            unsigned j;
+            for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
+                if (static_cast<unsigned>(lane) < cnt) {
+                    src[w][0][lane] = xs[j];
+                    src[w][1][lane] = xs[n + j];
+                    src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
                 }
-            __syncwarp();
-        }
-        if (g > 1) {
-            red[w][0][lane] = ax, red[w][1][lane] = ay, red[w][2][lane] = az;
-            __syncwarp();
-            if (grp == 0)
-                for (int q = 1; q < g; ++q) ax += red[w][0][t + q * nt], ay += red[w][1][t + q * nt], az += red[w][2][t + q * nt];
-            __syncwarp();
-        }
-        if (grp == 0) {
-            if (it.ns == 1) {
-                nearv[i] = Gm * ax;
-                nearv[n + i] = Gm * ay;
-                nearv[2 * static_cast<size_t>(n) + i] = Gm * az;
-            } else {
-                double *o = part + static_cast<size_t>(it.pslot) * 96;
+                __syncwarp();
+                if (tact)
+#pragma unroll 2
+                    for (unsigned k = grp; k < cnt; k += g) {
+                        const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
+                        double f;
+                        if (!rinv3(dx, dy, dz, soft, f)) {
+                            const double r2 = dx * dx + dy * dy + dz * dz + eps2;
+                            double ri = rsqrt(r2);
+                            if (!kSoft) ri = r2 > 0.0 ? ri : 0.0;
+                            f = ri * ri * ri;
+                        }
+                        ax += f * dx;
+                        ay += f * dy;
+                        az += f * dz;
+                    }
+                __syncwarp();
+            }
+            if (g > 1) {
+                red[w][0][lane] = ax, red[w][1][lane] = ay, red[w][2][lane] = az;
+                __syncwarp();
+                if (grp == 0)
+                    for (int q = 1; q < g; ++q) ax += red[w][0][t + q * nt], ay += red[w][1][t + q * nt], az += red[w][2][t + q * nt];
+                __syncwarp();
+            }
+            if (it.whole()) {
+                sum[w][0][lane] += ax, sum[w][1][lane] += ay, sum[w][2][lane] += az;
+            } else if (grp == 0) {
+                double *o = part + static_cast<size_t>(it.pslot + sl - it.sl) * 96;
                 o[t] = ax, o[32 + t] = ay, o[64 + t] = az;
             }
+        }
+        if (grp == 0 && it.whole()) {
+            nearv[i] = Gm * sum[w][0][lane];
+            nearv[n + i] = Gm * sum[w][1][lane];
+            nearv[2 * static_cast<size_t>(n) + i] = Gm * sum[w][2][lane];
         }
     }
 }
 
 // Sum the slices of every split chunk in slice order (deterministic).
 template <typename T>
-__global__ void k_p2p_combine(const int4 *__restrict__ chunks, const unsigned *counts, const T *__restrict__ part, T scale,
-                              T *__restrict__ nearv, unsigned n) {
+__global__ void k_p2p_combine(const int4 *__restrict__ chunks, const unsigned *counts, const LeafRec *__restrict__ recs,
+                              const T *__restrict__ part, T scale, T *__restrict__ nearv, unsigned n) {
     const unsigned nit = counts[5];
     for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nit * 32u; q += gridDim.x * blockDim.x) {
         const int4 w = chunks[q >> 5];
         const int t = static_cast<int>(q & 31u);
         const int ns = item_nslices(w.z);
-        if (ns <= 1 || item_slice(w.z) != 0 || t >= item_nt(w.z)) continue;
+        if (item_slice(w.z) != 0 || t >= item_nt(w.z) || ns <= recs[w.x].spi) continue;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             T s = 0;
@@ -356,8 +388,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
         ci = __shfl_sync(0xffffffffu, ci, 0);
         if (ci >= nch) break;
         Item it(chunks[ci]);
-        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total
-        it.slice(rec.z);
+        const uint4 rec = reinterpret_cast<const uint4 *>(recs + it.li)[0];  // rng_off, rng_len, src_total, spi
+        const unsigned slice = recs[it.li].slice;
+        it.of_leaf(static_cast<int>(rec.w));
         const int nt = it.nt;
         const int g = 32 / nt;
         const int grp = lane / nt;
@@ -365,41 +398,45 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_phi(const int4 *__restri
         const bool tact = grp < g;
         const unsigned i = static_cast<unsigned>(it.t0 + t);
         const double tx = tact ? xs[i] : 0.0, ty = tact ? xs[n + i] : 0.0, tz = tact ? xs[2 * static_cast<size_t>(n) + i] : 0.0;
-        double pot = 0;
-        BatchCursor cur;
-        cur.start(ranges + rec.x, rec.y, it.v0, it.len, static_cast<unsigned>(lane));
-        unsigned j;
-        for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
-            if (static_cast<unsigned>(lane) < cnt) {
-                src[w][0][lane] = xs[j];
-                src[w][1][lane] = xs[n + j];
-                src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
-                sidx[w][lane] = j;
-            }
-            __syncwarp();
-            if (tact)
-                for (unsigned k = grp; k < cnt; k += g) {
-                    if (sidx[w][k] == i) continue;
-                    const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
-                    double f;
-                    if (!rinv1(dx, dy, dz, soft, f)) f = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
-                    pot += f;
+        double opot = 0;  // the finished slices' sums
+        for (int sl = it.sl; sl < it.se; ++sl) {
+            unsigned v0, len;
+            v0 = min(rec.z, static_cast<unsigned>(sl) * slice), len = min(slice, rec.z - v0);
+            double pot = 0;
+            BatchCursor cur;
+            cur.start(ranges + rec.x, rec.y, v0, len, static_cast<unsigned>(lane));
+            unsigned j;
+            for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
+                if (static_cast<unsigned>(lane) < cnt) {
+                    src[w][0][lane] = xs[j];
+                    src[w][1][lane] = xs[n + j];
+                    src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
+                    sidx[w][lane] = j;
                 }
-            __syncwarp();
+                __syncwarp();
+                if (tact)
+                    for (unsigned k = grp; k < cnt; k += g) {
+                        if (sidx[w][k] == i) continue;
+                        const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
+                        double f;
+                        if (!rinv1(dx, dy, dz, soft, f)) f = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+                        pot += f;
+                    }
+                __syncwarp();
+            }
+            if (g > 1) {
+                red[w][lane] = pot;
+                __syncwarp();
+                if (grp == 0)
+                    for (int q = 1; q < g; ++q) pot += red[w][t + q * nt];
+                __syncwarp();
+            }
+            if (it.whole())
+                opot += pot;
+            else if (grp == 0)
+                part[static_cast<size_t>(it.pslot + sl - it.sl) * 96 + t] = pot;
         }
-        if (g > 1) {
-            red[w][lane] = pot;
-            __syncwarp();
-            if (grp == 0)
-                for (int q = 1; q < g; ++q) pot += red[w][t + q * nt];
-            __syncwarp();
-        }
-        if (grp == 0) {
-            if (it.ns == 1)
-                phiv[i] = Gm * pot;
-            else
-                part[static_cast<size_t>(it.pslot) * 96 + t] = pot;
-        }
+        if (grp == 0 && it.whole()) phiv[i] = Gm * opot;
     }
 }
 
@@ -414,14 +451,14 @@ __global__ void k_scale_by_system(T *__restrict__ v, unsigned n, int comps, cons
     }
 }
 
-__global__ void k_p2p_phi_combine(const int4 *__restrict__ chunks, const unsigned *counts, const double *__restrict__ part,
-                                  double Gm, double *__restrict__ phiv) {
+__global__ void k_p2p_phi_combine(const int4 *__restrict__ chunks, const unsigned *counts,
+                                  const LeafRec *__restrict__ recs, const double *__restrict__ part, double Gm, double *__restrict__ phiv) {
     const unsigned nit = counts[5];
     for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nit * 32u; q += gridDim.x * blockDim.x) {
         const int4 w = chunks[q >> 5];
         const int t = static_cast<int>(q & 31u);
         const int ns = item_nslices(w.z);
-        if (ns <= 1 || item_slice(w.z) != 0 || t >= item_nt(w.z)) continue;
+        if (item_slice(w.z) != 0 || t >= item_nt(w.z) || ns <= recs[w.x].spi) continue;
         double s = 0;
         for (int k = 0; k < ns; ++k) s += part[static_cast<size_t>(w.w + k) * 96 + t];
         phiv[w.y + t] = Gm * s;
@@ -437,7 +474,7 @@ void near_potential(Workspace &ws, double *phiv) {
     k_p2p_phi<<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.xs,
                                                 static_cast<double *>(ws.part), Gm, ws.eps * ws.eps,
                                                 soft_int(ws.eps * ws.eps), phiv, ws.n);
-    k_p2p_phi_combine<<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, static_cast<const double *>(ws.part), Gm, phiv);
+    k_p2p_phi_combine<<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.leaf_rec, static_cast<const double *>(ws.part), Gm, phiv);
     ws.launches += 2;
     if (ws.forest()) {
         k_scale_by_system<double><<<gs, 256, 0, ws.st>>>(phiv, ws.n, 1, ws.psys, ws.info);
@@ -460,10 +497,17 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
         const float Gm = ws.forest() ? 1.0f : static_cast<float>(ws.G * ws.m);  // a forest scales in p2p_finish
         auto *o = static_cast<float *>(ws.nearf);
         auto *pf = static_cast<float *>(ws.part);
-#define GB_P2P32(NW, SF)                                                                                             \
-    full_shared(k_p2p_f32<NW, SF>);                                                                                  \
-    k_p2p_f32<NW, SF><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.ph, \
+#define GB_P2P32_(NW, SF, MU)                                                                                           \
+    full_shared(k_p2p_f32<NW, SF, MU>);                                                                                  \
+    k_p2p_f32<NW, SF, MU><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.ph, \
                                                         ws.pl, pf, Gm, eps2, o, ws.n)
+#define GB_P2P32(NW, SF)             \
+    if (forest) {                    \
+        GB_P2P32_(NW, SF, true);     \
+    } else {                         \
+        GB_P2P32_(NW, SF, false);    \
+    }
+        const bool forest = ws.forest();
         if (ws.p2p_newton && soft) {
             GB_P2P32(true, true);
         } else if (ws.p2p_newton) {
@@ -474,6 +518,7 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
             GB_P2P32(false, false);
         }
 #undef GB_P2P32
+#undef GB_P2P32_
     } else {
         const double Gm = ws.forest() ? 1.0 : ws.G * ws.m, eps2 = ws.eps * ws.eps;
         auto *o = static_cast<double *>(ws.nearf);
@@ -497,10 +542,10 @@ void p2p_finish(Workspace &ws) {
     const bool forest = ws.forest();
     const double Gm = forest ? 1.0 : ws.G * ws.m;
     if (ws.mixed)
-        k_p2p_combine<float><<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, static_cast<const float *>(ws.part),
+        k_p2p_combine<float><<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.leaf_rec, static_cast<const float *>(ws.part),
                                                     static_cast<float>(Gm), static_cast<float *>(ws.nearf), ws.n);
     else
-        k_p2p_combine<double><<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, static_cast<const double *>(ws.part), Gm,
+        k_p2p_combine<double><<<gs, 256, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.leaf_rec, static_cast<const double *>(ws.part), Gm,
                                                      static_cast<double *>(ws.nearf), ws.n);
     ws.launches += 1;
     if (forest) {

@@ -37,9 +37,43 @@ constexpr int kTB = 256;
 // pipe instead of GB300's narrow FP64 pipe.
 __device__ __forceinline__ long long ord_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
 
-__global__ void k_bbox_partial(const double *__restrict__ x, unsigned n, double *__restrict__ part, TreeInfo *info) {
+// Root box (padded by Problem::OCTREE_WIDTH_PADDING, problem.hpp:167) and the
+// key parameters derived from it, from the particles' min and max; by one warp,
+// axis a on lane a (the divisions of one thread took ~10 us on the FP64 pipe).
+__device__ void set_root_box(TreeInfo *info, double mn, double mx) {
+    const double pad = 1e-5;
+    const int lane = threadIdx.x & 31, a = lane < 3 ? lane : 0;
+    const double lo = mn - pad, hi = mx + pad, H = hi - lo;
+    const double scale = ldexp(1.0, kMaxLevel) / H;
+    // Recursive FP64 midpoints stray from the ideal ones by at most
+    // 21/2 ulp(max|bound|) and u = (x - lo) 2^21 / H carries about one more
+    // ulp; in key units that is < 12 * 2^-52 * 2^21 * max|bound| / H.
+    const double big = fmax(fabs(lo), fabs(hi));
+    double margin = fmax(0.0, 64.0 * ldexp(big / H, -31) + ldexp(1.0, -30)), S = fmax(0.0, H);
+    const double m1 = __shfl_sync(0xffffffffu, margin, 1), m2 = __shfl_sync(0xffffffffu, margin, 2);
+    const double s1 = __shfl_sync(0xffffffffu, S, 1), s2 = __shfl_sync(0xffffffffu, S, 2);
+    margin = fmax(fmax(margin, m1), m2), S = fmax(fmax(S, s1), s2);
+    if (lane < 3) {
+        info->root_min[a] = lo, info->root_max[a] = hi, info->H[a] = H;
+        info->key_scale[a] = scale;
+        const double scale32 = ldexp(scale, 32);
+        info->key_scale32[a] = scale32;
+        info->key_off32[a] = -lo * scale32;
+        info->root_c[a] = (lo + hi) / 2;
+    }
+    if (lane == 0) {
+        info->S = S, info->key_margin = margin;
+        info->key_mfrac = static_cast<unsigned long long>(ceil(ldexp(margin, 32))) + 1;
+    }
+}
+
+// Bounding box: every block's minima and maxima (as ordered integers) into
+// part[6][blocks]; the last block to finish (counted in counts[11]) reduces them
+// and sets the root box. Min and max do not depend on the order.
+__global__ void __launch_bounds__(kTB) k_bbox(const double *__restrict__ x, unsigned n, long long *__restrict__ part,
+                                              unsigned *counts, TreeInfo *info) {
     const long long kmax = ord_key(__double_as_longlong(DBL_MAX)), kmin = ord_key(__double_as_longlong(-DBL_MAX));
-    long long kn[3] = {kmax, kmax, kmax}, kx[3] = {kmin, kmin, kmin};
+    long long k6[6] = {kmax, kmax, kmax, kmin, kmin, kmin};  // minima, maxima
     bool bad = false;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #pragma unroll
@@ -48,95 +82,53 @@ __global__ void k_bbox_partial(const double *__restrict__ x, unsigned n, double 
             const bool fin = ((b >> 52) & 0x7ff) != 0x7ff;  // non-finite values are skipped, as fmin / fmax do NaN
             bad |= !fin;
             const long long k = ord_key(b);
-            if (fin) kn[a] = min(kn[a], k), kx[a] = max(kx[a], k);
+            if (fin) k6[a] = min(k6[a], k), k6[3 + a] = max(k6[3 + a], k);
         }
     }
     if (bad) atomicOr(&info->err, kDevNonFinite);
-    double mn[3], mx[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        // +-0 compare equal as doubles: either is the box's bound (the padding makes them the same)
-        mn[a] = __longlong_as_double(ord_key(kn[a]));
-        mx[a] = __longlong_as_double(ord_key(kx[a]));
-    }
-    __shared__ double red[6][32];
+    __shared__ long long red[6][kTB / 32];
+    __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto block_reduce = [&]() {  // red[q][warp]
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) {
-            mn[a] = fmin(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-            mx[a] = fmax(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+        for (int q = 0; q < 6; ++q) {
+            for (int o = 16; o; o >>= 1) {
+                const long long u = __shfl_xor_sync(0xffffffffu, k6[q], o);
+                k6[q] = q < 3 ? min(k6[q], u) : max(k6[q], u);
+            }
+            if (lane == 0) red[q][w] = k6[q];
         }
-        if (lane == 0) red[a][w] = mn[a], red[3 + a][w] = mx[a];
-    }
+        __syncthreads();
+    };
+    auto of_warps = [&](int q) {
+        long long r = red[q][0];
+        for (int k = 1; k < kTB / 32; ++k) r = q < 3 ? min(r, red[q][k]) : max(r, red[q][k]);
+        return r;
+    };
+    block_reduce();
+    if (threadIdx.x < 6) part[threadIdx.x * gridDim.x + blockIdx.x] = of_warps(threadIdx.x);
+    __threadfence();
     __syncthreads();
-    if (threadIdx.x < 6) {
-        const int q = threadIdx.x;
-        double r = q < 3 ? DBL_MAX : -DBL_MAX;
-        for (int k = 0; k < static_cast<int>(blockDim.x >> 5); ++k) r = q < 3 ? fmin(r, red[q][k]) : fmax(r, red[q][k]);
-        part[q * gridDim.x + blockIdx.x] = r;
-    }
-}
-
-__device__ void set_root_box(TreeInfo *info, const double *mn, const double *mx);
-
-// One block of kTB threads; min and max do not depend on the order of the
-// partials, so the parallel reduction gives the same box as a serial one.
-__global__ void __launch_bounds__(kTB) k_bbox_final(const double *__restrict__ part, int nb, TreeInfo *info) {
-    __shared__ double red[6][kTB / 32];
-    double v[6];
+    if (threadIdx.x == 0) last = atomicAdd(counts + 11, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
 #pragma unroll
-    for (int a = 0; a < 3; ++a) v[a] = DBL_MAX, v[3 + a] = -DBL_MAX;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    for (int q = 0; q < 6; ++q) k6[q] = q < 3 ? kmax : kmin;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) v[a] = fmin(v[a], part[a * nb + b]), v[3 + a] = fmax(v[3 + a], part[(3 + a) * nb + b]);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        for (int o = 16; o; o >>= 1) {
-            const double u = __shfl_xor_sync(0xffffffffu, v[q], o);
-            v[q] = q < 3 ? fmin(v[q], u) : fmax(v[q], u);
+        for (int q = 0; q < 6; ++q) {
+            const long long u = __ldcg(part + q * gridDim.x + b);
+            k6[q] = q < 3 ? min(k6[q], u) : max(k6[q], u);
         }
-        if (lane == 0) red[q][w] = v[q];
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    double mn[3], mx[3];
-    for (int a = 0; a < 3; ++a) {
-        mn[a] = DBL_MAX, mx[a] = -DBL_MAX;
-        for (int k = 0; k < static_cast<int>(blockDim.x >> 5); ++k) mn[a] = fmin(mn[a], red[a][k]), mx[a] = fmax(mx[a], red[3 + a][k]);
-    }
-    set_root_box(info, mn, mx);
+    block_reduce();
+    if (w != 0) return;
+    const int a = lane < 3 ? lane : 0;
+    // +-0 compare equal as doubles: either is the box's bound (the padding makes them the same)
+    set_root_box(info, __longlong_as_double(ord_key(of_warps(a))), __longlong_as_double(ord_key(of_warps(3 + a))));
 }
 
-// Root box (padded by Problem::OCTREE_WIDTH_PADDING, problem.hpp:167) and
-// the key parameters derived from it, from the particles' min and max.
-__device__ void set_root_box(TreeInfo *info, const double *mn, const double *mx) {
-    const double pad = 1e-5;
-    double S = 0, margin = 0;
-    for (int a = 0; a < 3; ++a) {
-        info->root_min[a] = mn[a] - pad;
-        info->root_max[a] = mx[a] + pad;
-        info->H[a] = info->root_max[a] - info->root_min[a];
-        S = fmax(S, info->H[a]);
-        info->key_scale[a] = ldexp(1.0, kMaxLevel) / info->H[a];
-        // Recursive FP64 midpoints stray from the ideal ones by at most
-        // 21/2 ulp(max|bound|) and u = (x - lo) 2^21 / H carries about one more
-        // ulp; in key units that is < 12 * 2^-52 * 2^21 * max|bound| / H.
-        const double big = fmax(fabs(info->root_min[a]), fabs(info->root_max[a]));
-        margin = fmax(margin, 64.0 * ldexp(big / info->H[a], -31) + ldexp(1.0, -30));
-    }
-    info->S = S;
-    info->key_margin = margin;
-    for (int a = 0; a < 3; ++a) {
-        info->key_scale32[a] = ldexp(info->key_scale[a], 32);
-        info->key_off32[a] = -info->root_min[a] * info->key_scale32[a];
-        info->root_c[a] = (info->root_min[a] + info->root_max[a]) / 2;
-    }
-    info->key_mfrac = static_cast<unsigned long long>(ceil(ldexp(margin, 32))) + 1;
-}
-
-// Forest: one block per system, the same box as k_bbox_partial/final give
+// Forest: one block per system, the same box as k_bbox gives
 // for that system alone (min and max are exact), plus the system's particle
 // mass and G m. An empty system gets the box of the origin (no particle
 // uses it).
@@ -169,17 +161,14 @@ __global__ void __launch_bounds__(kTB) k_bbox_sys(const double *__restrict__ x, 
         if (lane == 0) red[a][w] = kn[a], red[3 + a][w] = kx[a];
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    double mn[3], mx[3];
-    for (int a = 0; a < 3; ++a) {
-        long long lo = red[a][0], hi = red[3 + a][0];
-        for (int k = 1; k < kTB / 32; ++k) lo = min(lo, red[a][k]), hi = max(hi, red[3 + a][k]);
-        // +-0 compare equal as doubles: either is the bound (the padding makes them the same)
-        mn[a] = e > b ? __longlong_as_double(ord_key(lo)) : 0.0;
-        mx[a] = e > b ? __longlong_as_double(ord_key(hi)) : 0.0;
-    }
+    if (w != 0) return;
+    const int a = lane < 3 ? lane : 0;
+    long long lo = red[a][0], hi = red[3 + a][0];
+    for (int k = 1; k < kTB / 32; ++k) lo = min(lo, red[a][k]), hi = max(hi, red[3 + a][k]);
     TreeInfo *si = info + sidx;
-    set_root_box(si, mn, mx);
+    // +-0 compare equal as doubles: either is the bound (the padding makes them the same)
+    set_root_box(si, e > b ? __longlong_as_double(ord_key(lo)) : 0.0, e > b ? __longlong_as_double(ord_key(hi)) : 0.0);
+    if (lane != 0) return;
     si->m = sys_par[sidx].x;
     si->gm = sys_par[sidx].y;
 }
@@ -765,15 +754,15 @@ __global__ void k_lists(const uint64_t *__restrict__ ent, const unsigned *counts
 // ancestors from the root down, then its own (the inherited list of
 // solver_ref.hpp:126 followed by the cell's additions). Each entry is a
 // subtree, i.e. a contiguous particle range in tree order.
-__device__ __forceinline__ unsigned leaf_slice(int c, unsigned slice, bool fp32, unsigned n, const unsigned *seg,
-                                               const int *c_sys) {
-    return slice_length(seg ? seg[c_sys[c] + 1] - seg[c_sys[c]] : n, slice, fp32);
+// particles of leaf c's system
+__device__ __forceinline__ unsigned leaf_system_n(int c, unsigned n, const unsigned *seg, const int *c_sys) {
+    return seg ? seg[c_sys[c] + 1] - seg[c_sys[c]] : n;
 }
 
 __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
                             const int *__restrict__ c_begin, const int *__restrict__ c_end,
                             const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt, unsigned *rng_cnt,
-                            unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, bool fp32, unsigned n,
+                            unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, unsigned n,
                             const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
     const unsigned NL = counts[3];
     for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < NL; li += gridDim.x * blockDim.x) {
@@ -790,9 +779,12 @@ __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *coun
                 }
             }
         rng_cnt[li] = tot;
-        const unsigned ns = nt > 0 ? static_cast<unsigned>(slice_count(srcs, leaf_slice(c, slice, fp32, n, seg, c_sys))) : 1u;
-        chunk_cnt[li] = static_cast<unsigned>(chunk_count(nt)) * ns;
-        part_cnt[li] = ns > 1 ? static_cast<unsigned>(chunk_count(nt)) * ns : 0u;
+        const unsigned nsys = leaf_system_n(c, n, seg, c_sys);
+        const unsigned ll = leaf_slice(srcs, nsys, slice);
+        const int ns = nt > 0 ? slice_count(srcs, ll) : 1;
+        const int spi = seg ? slices_per_item(n, slice, ll) : 1, nit = (ns + spi - 1) / spi;
+        chunk_cnt[li] = static_cast<unsigned>(chunk_count(nt) * nit);
+        part_cnt[li] = nit > 1 ? static_cast<unsigned>(chunk_count(nt) * ns) : 0u;
         src_total[li] = static_cast<unsigned>(srcs < 0xffffffffull ? srcs : 0xffffffffull);
     }
 }
@@ -808,7 +800,7 @@ __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, uns
                            const unsigned *__restrict__ rng_off, LeafRec *leaf_rec, const double *__restrict__ c_ctr,
                            uint2 *ranges,
                            const unsigned *__restrict__ chunk_off, int4 *chunks, const unsigned *__restrict__ src_total,
-                           const unsigned *__restrict__ part_off, unsigned part_cap, TreeInfo *info, unsigned slice, bool fp32, unsigned n,
+                           const unsigned *__restrict__ part_off, unsigned part_cap, TreeInfo *info, unsigned slice, unsigned n,
                            const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         counts[7] = counts[5];  // requested sizes, kept for the host when they overflow
@@ -862,27 +854,30 @@ __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, uns
                 overflow = true;
             ++k;
         }
+        const unsigned nsys = leaf_system_n(c, n, seg, c_sys);
+        const unsigned ll = leaf_slice(src_total[li], nsys, slice);
+        const int spi = seg ? slices_per_item(n, slice, ll) : 1;
         {
             const RootC cc = leaf_centre(c_ctr, c, info + cell_system(c_sys, c));
             LeafRec r{};
             r.rng_off = base, r.rng_len = overflow ? 0u : k;  // never let P2P read past the buffer
-            r.src_total = src_total[li];
+            r.src_total = src_total[li], r.spi = spi, r.slice = ll;
             r.hx = cc.hx, r.hy = cc.hy, r.hz = cc.hz, r.lx = cc.lx, r.ly = cc.ly, r.lz = cc.lz;
             leaf_rec[li] = r;
         }
         const unsigned cb = chunk_off[li];
         const int nch = chunk_count(e - b);
-        const int ns = slice_count(src_total[li], leaf_slice(c, slice, fp32, n, seg, c_sys));
+        const int ns = slice_count(src_total[li], ll), nit = (ns + spi - 1) / spi;
         for (int q = 0; q < nch; ++q) {
             int off, len;
             chunk_at(e - b, q, off, len);
-            for (int sl = 0; sl < ns; ++sl) {
-                const unsigned it = cb + static_cast<unsigned>(q * ns + sl);
-                // split items keep their partial sums in part[pslot]
-                const unsigned pslot = ns > 1 ? part_off[li] + static_cast<unsigned>(q * ns + sl) : 0xffffffffu;
-                if (ns > 1 && pslot >= part_cap) overflow = true;
+            for (int k = 0; k < nit; ++k) {
+                const unsigned it = cb + static_cast<unsigned>(q * nit + k);
+                // items of a split list keep their slices' partial sums in part[pslot ..]
+                const unsigned pslot = nit > 1 ? part_off[li] + static_cast<unsigned>(q * ns + k * spi) : 0xffffffffu;
+                if (nit > 1 && pslot + static_cast<unsigned>(min(spi, ns - k * spi)) > part_cap) overflow = true;
                 if (it < ch_cap)
-                    chunks[it] = make_int4(static_cast<int>(li), b + off, item_pack(len, sl, ns), static_cast<int>(pslot));
+                    chunks[it] = make_int4(static_cast<int>(li), b + off, item_pack(len, k * spi, ns), static_cast<int>(pslot));
                 else
                     overflow = true;
             }
@@ -1045,33 +1040,39 @@ void forest_tiles(Workspace &ws, int rows) {
     ws.launches += 5;
 }
 
+void tree_box(Workspace &ws) {
+    timer_begin(ws, kTTree);
+    k_eval_begin<<<1, 128, 0, ws.st>>>(ws.info, ws.d_counts, ws.n, ws.queue);
+    if (ws.forest())
+        k_bbox_sys<<<ws.nsys, kTB, 0, ws.st>>>(ws.x, ws.n, ws.seg, ws.sys_par, ws.info);
+    else
+        k_bbox<<<capped_grid(2 * ws.num_sms, ceil_div(ws.n, 2 * kTB)), kTB, 0, ws.st>>>(
+            ws.x, ws.n, reinterpret_cast<long long *>(ws.bbox_part), ws.d_counts, ws.info);
+    ws.launches += 2;
+    timer_end(ws, kTTree);
+}
+
 void build_tree(Workspace &ws) {
     const unsigned n = ws.n;
     cudaStream_t st = ws.st;
     timer_begin(ws, kTTree);
-    k_eval_begin<<<1, 128, 0, st>>>(ws.info, ws.d_counts, n, ws.queue);
     const bool forest = ws.forest();
     if (!forest) {
-        const int nb = 2 * ws.num_sms;
-        double *part = ws.bbox_part;
-        k_bbox_partial<<<nb, kTB, 0, st>>>(ws.x, n, part, ws.info);
-        k_bbox_final<<<1, kTB, 0, st>>>(part, nb, ws.info);
         const int kbit = 3 * (kMaxLevel - ws.sort_levels);
         k_keys<<<grid_for(n, kTB), kTB, 0, st>>>(ws.x, n, ws.info, ws.keys0, ws.perm0,
                                                  sort_zero_plan(ws.sort, n, kbit, 3 * kMaxLevel));
-        ws.launches += 4;
+        ws.launches += 1;
         const int res = radix_sort_u64(ws.keys0, ws.perm0, ws.keys1, ws.perm1, n, nullptr, kbit, 3 * kMaxLevel, ws.sort, st,
                                        &ws.launches, &ws.info->err, kDevTimeout, true, ws.sort_spin_max);
         ws.keys = res ? ws.keys1 : ws.keys0;
         ws.perm = res ? ws.perm1 : ws.perm0;
     } else {
-        // every system's box, then one sort of (system, key prefix) words and
+        // one sort of (system, key prefix) words and
         // the Morton keys gathered into sorted order (into the other key buffer)
-        k_bbox_sys<<<ws.nsys, kTB, 0, st>>>(ws.x, n, ws.seg, ws.sys_par, ws.info);
         const int wbits = 3 * ws.sort_levels + ws.sys_bits;
         k_keys_forest<<<grid_for(n, kTB), kTB, 0, st>>>(ws.x, n, ws.info, ws.psys, ws.sort_levels, ws.keys0, ws.perm0,
                                                         ws.mkeys, sort_zero_plan(ws.sort, n, 0, wbits));
-        ws.launches += 3;
+        ws.launches += 1;
         const int res = radix_sort_u64(ws.keys0, ws.perm0, ws.keys1, ws.perm1, n, nullptr, 0, wbits, ws.sort, st,
                                        &ws.launches, &ws.info->err, kDevTimeout, true, ws.sort_spin_max);
         ws.perm = res ? ws.perm1 : ws.perm0;
@@ -1127,7 +1128,7 @@ void build_tree(Workspace &ws) {
                                 forest ? ws.c_sys : nullptr, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                                 reinterpret_cast<unsigned long long *>(&ws.info->m2l_pairs));
     k_rng_count<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
-                                    ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, ws.mixed, n, seg, forest ? ws.c_sys : nullptr);
+                                    ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
     {  // range, work-item and partial-slot offsets per leaf, one scan sequence
         ScanSet sc{};
         sc.in[0] = ws.rng_cnt, sc.out[0] = ws.rng_off, sc.total[0] = ws.d_counts + 4;
@@ -1137,7 +1138,7 @@ void build_tree(Workspace &ws) {
     }
     k_rng_fill<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
                                    ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.leaf_rec, ws.c_ctr, ws.ranges, ws.chunk_off, ws.chunks,
-                                   ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, ws.mixed, n, seg, forest ? ws.c_sys : nullptr);
+                                   ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
     ws.launches += 9;
     timer_end(ws, kTTree);
 }

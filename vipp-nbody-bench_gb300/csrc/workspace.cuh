@@ -35,8 +35,10 @@ enum TimerClass { kTTree = 0, kTOps = 1, kTUp = 2, kTM2L = 3, kTDown = 4, kTP2P 
 // in one read (and converts no FP64 centre: 15 operations on the narrow pipe).
 struct alignas(16) LeafRec {
     unsigned rng_off, rng_len, src_total;
+    int spi;  // slices per work item
+    unsigned slice;  // sources per slice
     float hx, hy, hz, lx, ly, lz;
-    float pad_[3];
+    float pad_;
 };
 
 struct Workspace {
@@ -53,6 +55,8 @@ struct Workspace {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t st3 = nullptr;         // accurate mode: the softening correction, concurrent with the far field
     cudaEvent_t ev_fork3 = nullptr, ev_join3 = nullptr;
+    cudaStream_t st4 = nullptr;         // operators, concurrent with the tree build
+    cudaEvent_t ev_box = nullptr, ev_ops = nullptr;
     bool serial = false;                // near field on st after the far field
     int sort_levels = 10;               // key levels the radix sort orders (grown on demand, up to 21)
     unsigned sort_spin_max = kSortSpinMax;  // look-back polls before a wait gives up (tests lower it)
@@ -174,7 +178,8 @@ struct Workspace {
     TreeInfo *info = nullptr;
     unsigned *d_counts = nullptr;  // [kNumCounts]: 0 n, 1 S, 2 C, 3 leaves, 4 ranges, 5 items,
                                    // 6 S requested, 7 items requested, 8 partial slots,
-                                   // 9 key levels a deeper sort needs (0: enough)
+                                   // 9 key levels a deeper sort needs (0: enough),
+                                   // 11 blocks done with the bounding box
     TreeInfo *h_info = nullptr;    // pinned mirror
 
     SortTemp sort;
@@ -213,17 +218,20 @@ constexpr int kOpL2L = 351;  // op index of L2L octant 0
 constexpr int kNumOps = 359;
 
 // stages (all asynchronous on ws.st)
-void build_tree(Workspace &ws);               // bbox, keys, sort, cells, leaves, lists, near-field ranges
+void tree_box(Workspace &ws);                 // start of an evaluation: counters, root box
+void build_tree(Workspace &ws);               // keys, sort, cells, leaves, lists, near-field ranges
 void forest_tiles(Workspace &ws, int rows);   // forest: M2M/L2L tiles and M2L tiles of `rows` octets per system
 void build_operators(Workspace &ws);          // 359 translation matrices for the current root box
 size_t m2l_table_bytes(int p);
 inline size_t zf_table_floats(int p) { return static_cast<size_t>(kNumOps) * (2 * p + 1) * (2 * p + 1); }  // per system
 void build_m2l_table(Workspace &ws);          // fill m2l_tab for ws.p (once per p, outside step graphs)
-void upward_pass(Workspace &ws);              // P2M + M2M
+void p2m_pass(Workspace &ws);
+void m2m_pass(Workspace &ws);
 void m2l_pass(Workspace &ws);                 // M2L into L (CUDA cores, FP32)
 void m2l_pass_f64(Workspace &ws);             // M2L into L (FP64)
 unsigned m2l_f64_tiles(const Workspace &ws);  // bound of the tiles of ws.c_cap cells
 size_t m2l_f64_part_doubles(int p);           // class-group sums of one tile
+void m2l_tc_images(Workspace &ws);            // operator images of the tensor-core M2L
 void m2l_pass_tc(Workspace &ws);              // M2L into L (tensor cores, mixed)
 bool m2l_tc_supported(int p);
 size_t m2l_tc_image_floats(int p);
