@@ -754,31 +754,81 @@ __global__ void k_lists(const uint64_t *__restrict__ ent, const unsigned *counts
 // ancestors from the root down, then its own (the inherited list of
 // solver_ref.hpp:126 followed by the cell's additions). Each entry is a
 // subtree, i.e. a contiguous particle range in tree order.
+//
+// kLanes lanes per leaf, a lane per entry: a thread per leaf walked the ancestors'
+// lists entry by entry, a chain of ~100 dependent loads that took 30 us whatever the
+// tree's size (k_rng_fill; k_rng_count 11 to 15). A warp per leaf has the shortest
+// chain and is taken while one grid holds a warp for every leaf; beyond that the
+// instructions of idle lanes count, and 4 lanes are taken. Tree class per RK4 step,
+// 4 / 8 / 16 / 32 lanes: 3,001 particles 0.519 / 0.497 / 0.485 / 0.482 ms; 100,003
+// 0.853 / 0.830 / 0.820 / 0.811; 4M 4.07 / 4.12 / 4.26 / 4.52; 16M 14.5 / 14.9 /
+// 15.5 / 16.6 (a thread per leaf: 0.62, 0.92, 4.03 and 14.7 or more).
+constexpr int kLeafLanesSmall = 32, kLeafLanesLarge = 4;
+constexpr int kLeafBatch = 4;  // ranges a lane has in flight
+constexpr int kLeafThreads = 256;
+
+struct LeafEntries {  // the near-field entries of a leaf; a group of lanes of one warp per leaf
+    int2 *anc;   // ancestor j counted from the leaf up: cell, entries up to and with it
+    int total;   // entries
+    int most;    // the largest total of the warp's leaves
+    int j;       // ancestor of this lane's next entry
+    // c < 0: no leaf
+    __device__ __forceinline__ LeafEntries(int2 *sh, int c, const int *__restrict__ c_parent, const int *__restrict__ p2p_cnt,
+                                           int gl)
+        : anc(sh), total(0), j(0) {
+        int na = 0;
+        for (int a = c; a >= 0 && na <= kMaxLevel; a = c_parent[a], ++na) {
+            total += p2p_cnt[a];
+            if (gl == 0) anc[na] = make_int2(a, total);
+        }
+        j = max(na - 1, 0);
+        most = __reduce_max_sync(0xffffffffu, total);
+        __syncwarp();
+    }
+    // particle range of entry k, root's entries first (empty past the last); k ascending per lane
+    __device__ __forceinline__ uint2 range(int k, const int *__restrict__ p2p_own, const int *__restrict__ c_begin,
+                                           const int *__restrict__ c_end) {
+        if (k >= total) return make_uint2(0, 0);
+        int2 a = anc[j];
+        while (k >= total - (j > 0 ? anc[j - 1].y : 0)) a = anc[--j];
+        const int u = p2p_own[static_cast<size_t>(a.x) * kNbrCap + (k - (total - a.y))];
+        return make_uint2(static_cast<unsigned>(c_begin[u]), static_cast<unsigned>(c_end[u]));
+    }
+};
+
 // particles of leaf c's system
 __device__ __forceinline__ unsigned leaf_system_n(int c, unsigned n, const unsigned *seg, const int *c_sys) {
     return seg ? seg[c_sys[c] + 1] - seg[c_sys[c]] : n;
 }
 
-__global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
+template <int kLanes>
+__global__ void __launch_bounds__(kLeafThreads) k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
                             const int *__restrict__ c_begin, const int *__restrict__ c_end,
                             const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt, unsigned *rng_cnt,
                             unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, unsigned n,
                             const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
+    __shared__ int2 anc[kLeafThreads / kLanes][kMaxLevel + 1];
     const unsigned NL = counts[3];
-    for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < NL; li += gridDim.x * blockDim.x) {
-        const int c = leaves[li];
-        const int nt = c_end[c] - c_begin[c];
-        unsigned tot = 0;
+    const int gl = threadIdx.x % kLanes, group = threadIdx.x / kLanes;
+    constexpr unsigned kGroups = kLeafThreads / kLanes;
+    for (unsigned l0 = blockIdx.x * kGroups; l0 < NL; l0 += gridDim.x * kGroups) {
+        const unsigned li = l0 + group;
+        const int c = li < NL ? leaves[li] : -1;
+        const int nt = c >= 0 ? c_end[c] - c_begin[c] : 0;
         unsigned long long srcs = 0;
-        if (nt > 0)
-            for (int a = c; a >= 0; a = c_parent[a]) {
-                tot += static_cast<unsigned>(p2p_cnt[a]);
-                for (int q = 0; q < p2p_cnt[a]; ++q) {
-                    const int u = p2p_own[static_cast<size_t>(a) * kNbrCap + q];
-                    srcs += static_cast<unsigned>(c_end[u] - c_begin[u]);
-                }
-            }
-        rng_cnt[li] = tot;
+        LeafEntries le(anc[group], nt > 0 ? c : -1, c_parent, p2p_cnt, gl);
+        for (int k0 = 0; k0 < le.most; k0 += kLanes * kLeafBatch) {
+            uint2 r[kLeafBatch];
+#pragma unroll
+            for (int q = 0; q < kLeafBatch; ++q) r[q] = le.range(k0 + q * kLanes + gl, p2p_own, c_begin, c_end);
+#pragma unroll
+            for (int q = 0; q < kLeafBatch; ++q) srcs += r[q].y - r[q].x;
+        }
+#pragma unroll
+        for (int o = kLanes / 2; o; o >>= 1) srcs += __shfl_xor_sync(0xffffffffu, srcs, o);
+        __syncwarp();  // anc is read
+        if (gl != 0 || li >= NL) continue;
+        rng_cnt[li] = static_cast<unsigned>(le.total);
         const unsigned nsys = leaf_system_n(c, n, seg, c_sys);
         const unsigned ll = leaf_slice(srcs, nsys, slice);
         const int ns = nt > 0 ? slice_count(srcs, ll) : 1;
@@ -794,7 +844,8 @@ __global__ void k_rng_count(const int *__restrict__ leaves, const unsigned *coun
 // address items whose partial-sum slot lies past part_cap, and the P2P kernels
 // run before the host sees the flag, grows the buffers and repeats the
 // evaluation).
-__global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
+template <int kLanes>
+__global__ void __launch_bounds__(kLeafThreads) k_rng_fill(const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
                            const int *__restrict__ c_parent, const int *__restrict__ c_begin, const int *__restrict__ c_end,
                            const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt,
                            const unsigned *__restrict__ rng_off, LeafRec *leaf_rec, const double *__restrict__ c_ctr,
@@ -809,82 +860,77 @@ __global__ void k_rng_fill(const int *__restrict__ leaves, unsigned *counts, uns
         counts[5] = over ? 0u : counts[5];
         info->n_p2p_chunks = static_cast<int>(counts[5]);
     }
+    __shared__ int2 anc[kLeafThreads / kLanes][kMaxLevel + 1];
     const unsigned NL = counts[3];
-    unsigned long long pairs = 0, nranges = 0;  // this thread's totals, added once per warp below
-    for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < NL; li += gridDim.x * blockDim.x) {
-        const int c = leaves[li];
-        const int b = c_begin[c], e = c_end[c];
-        if (e == b) {
-            continue;  // no work item names it
-        }
-        int anc[kMaxLevel + 2];
-        int na = 0;
-        for (int a = c; a >= 0 && na < kMaxLevel + 2; a = c_parent[a]) anc[na++] = a;
-        const unsigned base = rng_off[li];
-        unsigned k = 0;
-        unsigned long long srcs = 0;
-        uint2 last = make_uint2(0, 0);
-        bool have = false, overflow = false;
-        for (int t = na - 1; t >= 0; --t) {
-            const int a = anc[t];
-            for (int q = 0; q < p2p_cnt[a]; ++q) {
-                const int u = p2p_own[static_cast<size_t>(a) * kNbrCap + q];
-                const unsigned ub = static_cast<unsigned>(c_begin[u]), ue = static_cast<unsigned>(c_end[u]);
-                if (ue == ub) continue;
-                srcs += ue - ub;
-                if (have && last.y == ub) {
-                    last.y = ue;
-                } else {
-                    if (have) {
-                        if (base + k < r_cap)
-                            ranges[base + k] = last;
-                        else
-                            overflow = true;
-                        ++k;
-                    }
-                    last = make_uint2(ub, ue);
-                    have = true;
+    constexpr unsigned kGroups = kLeafThreads / kLanes;
+    constexpr unsigned kGroupMask = kLanes == 32 ? 0xffffffffu : (1u << (kLanes % 32)) - 1u;
+    const int gl = threadIdx.x % kLanes, group = threadIdx.x / kLanes;
+    const int glo = (threadIdx.x & 31) - gl;  // the group's first lane
+    const unsigned lower = (1u << gl) - 1u;
+    unsigned long long pairs = 0, nranges = 0;  // the group's first lane: its totals, added once per warp below
+    for (unsigned l0 = blockIdx.x * kGroups; l0 < NL; l0 += gridDim.x * kGroups) {
+        const unsigned li = l0 + group;
+        const int c = li < NL ? leaves[li] : -1;
+        const int b = c >= 0 ? c_begin[c] : 0, e = c >= 0 ? c_end[c] : 0;
+        LeafEntries le(anc[group], e > b ? c : -1, c_parent, p2p_cnt, gl);
+        const unsigned base = e > b ? rng_off[li] : 0;
+        // merged ranges: an entry that begins where the last non-empty one ended extends
+        // its range, which is open until the next one starts
+        unsigned nr = 0, open_end = 0;
+        for (int k0 = 0; k0 < le.most; k0 += kLanes * kLeafBatch) {
+            uint2 r[kLeafBatch];
+#pragma unroll
+            for (int q = 0; q < kLeafBatch; ++q) r[q] = le.range(k0 + q * kLanes + gl, p2p_own, c_begin, c_end);
+#pragma unroll
+            for (int q = 0; q < kLeafBatch; ++q) {
+                const bool some = r[q].y > r[q].x;
+                const unsigned mask = (__ballot_sync(0xffffffffu, some) >> glo) & kGroupMask, below = mask & lower;
+                const unsigned prev = __shfl_sync(0xffffffffu, r[q].y, glo + (below ? 31 - __clz(below) : 0));
+                const unsigned last = __shfl_sync(0xffffffffu, r[q].y, glo + (mask ? 31 - __clz(mask) : 0));
+                const bool starts = some && (below ? prev != r[q].x : nr == 0 || open_end != r[q].x);
+                const unsigned smask = (__ballot_sync(0xffffffffu, starts) >> glo) & kGroupMask;
+                if (starts) {
+                    const unsigned at = nr + __popc(smask & lower);
+                    if (base + at < r_cap) ranges[base + at].x = r[q].x;
+                    if (at > 0 && base + at - 1 < r_cap) ranges[base + at - 1].y = below ? prev : open_end;
                 }
+                nr += __popc(smask);
+                if (mask) open_end = last;
             }
         }
-        if (have) {
-            if (base + k < r_cap)
-                ranges[base + k] = last;
-            else
-                overflow = true;
-            ++k;
-        }
+        __syncwarp();  // anc is read
+        if (e == b) continue;  // no work item names it (no warp-wide step follows in this pass)
+        bool overflow = base + nr > r_cap;
+        if (gl == 0 && nr > 0 && !overflow) ranges[base + nr - 1].y = open_end;
         const unsigned nsys = leaf_system_n(c, n, seg, c_sys);
-        const unsigned ll = leaf_slice(src_total[li], nsys, slice);
+        const unsigned srcs = src_total[li], ll = leaf_slice(srcs, nsys, slice);
         const int spi = seg ? slices_per_item(n, slice, ll) : 1;
-        {
+        if (gl == 0) {
             const RootC cc = leaf_centre(c_ctr, c, info + cell_system(c_sys, c));
             LeafRec r{};
-            r.rng_off = base, r.rng_len = overflow ? 0u : k;  // never let P2P read past the buffer
-            r.src_total = src_total[li], r.spi = spi, r.slice = ll;
+            r.rng_off = base, r.rng_len = overflow ? 0u : nr;  // never let P2P read past the buffer
+            r.src_total = srcs, r.spi = spi, r.slice = ll;
             r.hx = cc.hx, r.hy = cc.hy, r.hz = cc.hz, r.lx = cc.lx, r.ly = cc.ly, r.lz = cc.lz;
             leaf_rec[li] = r;
         }
         const unsigned cb = chunk_off[li];
         const int nch = chunk_count(e - b);
-        const int ns = slice_count(src_total[li], ll), nit = (ns + spi - 1) / spi;
-        for (int q = 0; q < nch; ++q) {
+        const int ns = slice_count(srcs, ll), nit = (ns + spi - 1) / spi;
+        for (int w = gl; w < nch * nit; w += kLanes) {
+            const int q = w / nit, k = w - q * nit;
             int off, len;
             chunk_at(e - b, q, off, len);
-            for (int k = 0; k < nit; ++k) {
-                const unsigned it = cb + static_cast<unsigned>(q * nit + k);
-                // items of a split list keep their slices' partial sums in part[pslot ..]
-                const unsigned pslot = nit > 1 ? part_off[li] + static_cast<unsigned>(q * ns + k * spi) : 0xffffffffu;
-                if (nit > 1 && pslot + static_cast<unsigned>(min(spi, ns - k * spi)) > part_cap) overflow = true;
-                if (it < ch_cap)
-                    chunks[it] = make_int4(static_cast<int>(li), b + off, item_pack(len, k * spi, ns), static_cast<int>(pslot));
-                else
-                    overflow = true;
-            }
+            const unsigned it = cb + static_cast<unsigned>(w);
+            // items of a split list keep their slices' partial sums in part[pslot ..]
+            const unsigned pslot = nit > 1 ? part_off[li] + static_cast<unsigned>(q * ns + k * spi) : 0xffffffffu;
+            if (nit > 1 && pslot + static_cast<unsigned>(min(spi, ns - k * spi)) > part_cap) overflow = true;
+            if (it < ch_cap)
+                chunks[it] = make_int4(static_cast<int>(li), b + off, item_pack(len, k * spi, ns), static_cast<int>(pslot));
+            else
+                overflow = true;
         }
         if (overflow) atomicOr(&info->err, kDevCapacity);
-        pairs += static_cast<unsigned long long>(e - b) * srcs;
-        nranges += k;
+        if (gl == 0) pairs += static_cast<unsigned long long>(e - b) * srcs, nranges += nr;
     }
     // one atomic per warp and counter (per-leaf atomics on two addresses serialised the kernel)
 #pragma unroll
@@ -1127,8 +1173,13 @@ void build_tree(Workspace &ws) {
     k_lists<<<gs, 256, 0, st>>>(ws.ent, ws.d_counts, ws.split_cell, ws.info, ws.c_child, ws.c_path, ws.c_coord,
                                 forest ? ws.c_sys : nullptr, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                                 reinterpret_cast<unsigned long long *>(&ws.info->m2l_pairs));
-    k_rng_count<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
-                                    ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
+    // a warp per leaf while one grid has a warp for every leaf (figures at LeafEntries)
+    const unsigned full = static_cast<unsigned>(ws.num_sms) * 8;
+    const bool warp_each = ceil_div(ws.c_cap, kLeafThreads / kLeafLanesSmall) <= full;
+    const unsigned gl = warp_each ? ceil_div(ws.c_cap, kLeafThreads / kLeafLanesSmall)
+                                  : capped_grid(full, ceil_div(ws.c_cap, kLeafThreads / kLeafLanesLarge));
+    (warp_each ? k_rng_count<kLeafLanesSmall> : k_rng_count<kLeafLanesLarge>)<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
+        ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
     {  // range, work-item and partial-slot offsets per leaf, one scan sequence
         ScanSet sc{};
         sc.in[0] = ws.rng_cnt, sc.out[0] = ws.rng_off, sc.total[0] = ws.d_counts + 4;
@@ -1136,9 +1187,9 @@ void build_tree(Workspace &ws) {
         sc.in[2] = ws.part_cnt, sc.out[2] = ws.part_off, sc.total[2] = ws.d_counts + 8;
         scan_exclusive_multi(sc, 3, ws.c_cap, ws.d_counts + 3, ws.scan, st, &ws.launches);
     }
-    k_rng_fill<<<gs, kTB, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
-                                   ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.leaf_rec, ws.c_ctr, ws.ranges, ws.chunk_off, ws.chunks,
-                                   ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
+    (warp_each ? k_rng_fill<kLeafLanesSmall> : k_rng_fill<kLeafLanesLarge>)<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
+        ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.leaf_rec, ws.c_ctr, ws.ranges, ws.chunk_off, ws.chunks,
+        ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
     ws.launches += 9;
     timer_end(ws, kTTree);
 }
