@@ -371,21 +371,35 @@ __global__ void __launch_bounds__(128) k_soft_far(const int *__restrict__ leaves
 // records, then the parent's slots) in shared memory, then streams them in
 // batches of 32: each lane stages one record as its offset from the leaf
 // centre plus M, tr Q and Q (the next batch's records are loaded while the
-// current one is computed), and every lane applies the staged batch to up to
-// kTPL of the leaf's particles (targets lane, lane + 32, ...). Last, the
-// leaf-centre Taylor part is added and far = G (far + correction).
+// current one is computed). Last, the leaf-centre Taylor part is added and
+// far = G (far + correction).
+//
+// Paired path (FP32 field): the leaf's particles in the near field's chunks
+// (chunk_at), a chunk of t < 32 of them on floor(32 / t) groups of lanes that take
+// every so many-th record pair, up to kSoftChunks chunks per staged batch. Bound by
+// the FP32 pipe (58% active: 40 paired operations and 4 rsqrt per record pair, 16
+// warps per SM at 128 registers). With two targets per lane, lane and lane + 32, a
+// fifth of the lanes held no target (Plummer, s = 64): 1.96 -> 1.35 ms a launch at
+// 1,000,003 particles, p = 10, together with a block for every four leaves instead
+// of a grid of 8 per SM that each walked a fixed share (8.31 -> 7.50 ms per step of
+// four corrections).
 #ifndef GB_SOFT_TPL
-#define GB_SOFT_TPL 2  // targets per lane per pass (measured at 4M, p = 10: 2 -> 38.4, 4 -> 40.8, 8 -> 51.7 ms per step)
+#define GB_SOFT_TPL 2  // scalar path (FP64, potential): targets per lane per pass
+#endif
+#ifndef GB_SOFT_CHUNKS
+#define GB_SOFT_CHUNKS 3  // paired path: chunks per pass (1,000,003 Plummer, p = 10: 1 -> 8.47, 2 -> 7.57, 3 -> 7.50 ms per step)
 #endif
 #ifndef GB_SOFT_UNROLL
-#define GB_SOFT_UNROLL 4  // record pairs per unrolled step of the FP32 loop (4: 37.9 against 38.5 ms per step for 1)
+#define GB_SOFT_UNROLL 4  // record pairs per unrolled step (same: 2 -> 7.57, 3 -> 7.78, 4 -> 7.51, 5 -> 7.60)
 #endif
 #ifndef GB_SOFT_MIN_BLOCKS
-#define GB_SOFT_MIN_BLOCKS 1
+#define GB_SOFT_MIN_BLOCKS 4  // paired path: 128 registers (unbounded, 150: 7.73; 5 blocks, 96 registers: 7.74 to 7.99)
 #endif
 constexpr int kSoftWarps = 4;
 constexpr int kSoftTPL = GB_SOFT_TPL;
+constexpr int kSoftChunks = GB_SOFT_CHUNKS;
 constexpr int kSoftUnroll = GB_SOFT_UNROLL;
+constexpr int kSoftPairs = 16;  // record pairs per staged batch, one per two lanes
 constexpr int kSoftMaxSrc = 54 * 8 + 135 + 189;  // 756 records at most
 
 template <typename T>
@@ -486,18 +500,31 @@ __device__ __forceinline__ void soft_term_pair(const float4 *P, float2 ntx, floa
 // diagnostics): the scalar path, farphi[j] += correction (the far potential
 // is multiplied by G where near and far are added).
 template <typename T, bool kPhi = false>
-__global__ void __launch_bounds__(kSoftWarps * 32, GB_SOFT_MIN_BLOCKS) k_soft_near(
+__global__ void __launch_bounds__(kSoftWarps * 32, (sizeof(T) == 4 && !kPhi) ? GB_SOFT_MIN_BLOCKS : 1) k_soft_near(
     const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_begin, const int *__restrict__ c_end,
     const int *__restrict__ c_level, const int *__restrict__ c_parent, const int *__restrict__ c_child,
     const double *__restrict__ c_ctr, const TreeInfo *__restrict__ info, const int *__restrict__ m2l_src,
     const Mom<T> *__restrict__ mom, const Mom<T> *__restrict__ moct, const T *__restrict__ taylor,
     const double *__restrict__ xs, const float4 *__restrict__ ph, const float4 *__restrict__ pl, unsigned n, T e2, T G,
     T *__restrict__ far, double *__restrict__ farphi = nullptr, T *__restrict__ corr = nullptr) {
+    constexpr bool kPaired = sizeof(T) == 4 && !kPhi;
     __shared__ int list[kSoftWarps][kSoftMaxSrc + 32];
-    __shared__ __align__(16) SRec<T> batch[kSoftWarps][32];  // FP32: the paired layout (put_paired)
+    __shared__ __align__(16) SRec<T> batch[kSoftWarps][kPaired ? 1 : 32];
+    __shared__ __align__(16) float pairs[kSoftWarps][kPaired ? 24 * (kSoftPairs + 1) : 1];  // put_paired's layout
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned NL = counts[3];
     const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    auto put = [&](int j, T ax, T ay, T az) {
+        if (corr) {  // kept apart; soften_apply folds it into the far field
+            corr[j] = ax, corr[n + j] = ay, corr[2 * static_cast<size_t>(n) + j] = az;
+        } else {
+            far[j] = G * (far[j] + ax);
+            far[n + j] = G * (far[n + j] + ay);
+            far[2 * static_cast<size_t>(n) + j] = G * (far[2 * static_cast<size_t>(n) + j] + az);
+        }
+    };
+    if constexpr (kPaired)
+        if (lane < 24) pairs[w][24 * kSoftPairs + lane] = lane < 2 ? 1e10f : 0.f;  // the massless pair idle lanes take
     for (unsigned li = blockIdx.x * (blockDim.x >> 5) + w; li < NL; li += warps) {
         const int c = leaves[li];
         if (c_level[c] < 2) continue;  // warp-uniform
@@ -545,52 +572,87 @@ __global__ void __launch_bounds__(kSoftWarps * 32, GB_SOFT_MIN_BLOCKS) k_soft_ne
         }
         if (lane < 32) list[w][nsrc + lane] = INT_MIN;  // pad the last batch
         __syncwarp();
-        T tl[kTaylor];
-#pragma unroll
-        for (int k = 0; k < kTaylor; ++k) tl[k] = taylor[static_cast<size_t>(c) * kTaylor + k];
         const int b = c_begin[c], e = c_end[c];
-        for (int j0 = b; j0 < e; j0 += 32 * kSoftTPL) {
-            const int nq = min(kSoftTPL, (e - j0 + 31) / 32);  // warp-uniform
-            T ty[kSoftTPL][3], acc[kSoftTPL][3];
+        if constexpr (kPaired) {
+            float *pb = pairs[w];
+            const float4 *pb4 = reinterpret_cast<const float4 *>(pb);
+            const float2 e22 = make_float2(e2, e2);
+            const int nch = chunk_count(e - b);
+            for (int c0 = 0; c0 < nch; c0 += kSoftChunks) {
+                int j[kSoftChunks], g[kSoftChunks], grp[kSoftChunks], len[kSoftChunks];
+                float2 nt[kSoftChunks][3], a2[kSoftChunks][3];
 #pragma unroll
-            for (int q = 0; q < kSoftTPL; ++q) {
-                ty[q][0] = ty[q][1] = ty[q][2] = T(0);
-                acc[q][0] = acc[q][1] = acc[q][2] = T(0);
-                const int j = j0 + 32 * q + lane;
-                if (q < nq && j < e) rel_pos<T>(j, xs, n, ph, pl, cd, cc, ty[q]);
-            }
-            SRec<T> nxt;
-            if (nsrc > 0) stage<T>(mom, moct, list[w][lane], cc, nxt);
-            if constexpr (sizeof(T) == 4 && !kPhi) {
-                float *pb = reinterpret_cast<float *>(batch[w]);
-                const float4 *pb4 = reinterpret_cast<const float4 *>(pb);
-                const float2 e22 = make_float2(e2, e2);
-                float2 nt[kSoftTPL][3], a2[kSoftTPL][3];
-#pragma unroll
-                for (int q = 0; q < kSoftTPL; ++q)
+                for (int q = 0; q < kSoftChunks; ++q) {
+                    int off = 0;
+                    len[q] = 0, g[q] = 1;
+                    if (c0 + q < nch) {
+                        chunk_at(e - b, c0 + q, off, len[q]);
+                        g[q] = 32 / len[q];
+                    }
+                    grp[q] = len[q] ? lane / len[q] : 1;
+                    const int t = lane - grp[q] * len[q];
+                    j[q] = b + off + t;
+                    T ty[3] = {T(0), T(0), T(0)};
+                    if (grp[q] < g[q]) rel_pos<T>(j[q], xs, n, ph, pl, cd, cc, ty);
+                    if (grp[q] >= g[q]) grp[q] = kSoftPairs;
 #pragma unroll
                     for (int a = 0; a < 3; ++a)
-                        nt[q][a] = make_float2(-ty[q][a], -ty[q][a]), a2[q][a] = make_float2(0.f, 0.f);
+                        nt[q][a] = make_float2(-ty[a], -ty[a]), a2[q][a] = make_float2(0.f, 0.f);
+                }
+                SRec<T> nxt;
+                if (nsrc > 0) stage<T>(mom, moct, list[w][lane], cc, nxt);
                 for (int b0 = 0; b0 < nsrc; b0 += 32) {
                     put_paired(pb, lane, nxt);
                     __syncwarp();
                     if (b0 + 32 < nsrc) stage<T>(mom, moct, list[w][b0 + 32 + lane], cc, nxt);
                     // a padded batch's tail holds massless records whose terms are exactly zero
                     const int npairs = (min(32, nsrc - b0) + 1) >> 1;
-#pragma unroll kSoftUnroll
-                    for (int k = 0; k < npairs; ++k) {
 #pragma unroll
-                        for (int q = 0; q < kSoftTPL; ++q)
-                            if (q < nq)
-                                soft_term_pair(pb4 + 6 * k, nt[q][0], nt[q][1], nt[q][2], e22, a2[q][0], a2[q][1], a2[q][2]);
+                    for (int q = 0; q < kSoftChunks; ++q) {
+                        if (c0 + q >= nch) break;  // warp-uniform
+                        const int steps = (npairs + g[q] - 1) / g[q];
+                        int k = grp[q];
+#pragma unroll kSoftUnroll
+                        for (int i = 0; i < steps; ++i, k += g[q])
+                            soft_term_pair(pb4 + 6 * (k < npairs ? k : kSoftPairs), nt[q][0], nt[q][1], nt[q][2], e22, a2[q][0], a2[q][1],
+                                           a2[q][2]);
                     }
                     __syncwarp();
                 }
 #pragma unroll
-                for (int q = 0; q < kSoftTPL; ++q)
+                for (int q = 0; q < kSoftChunks; ++q) {
+                    if (c0 + q >= nch) break;
+                    T v[3];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) acc[q][a] = a2[q][a].x + a2[q][a].y;
-            } else {
+                    for (int a = 0; a < 3; ++a) {
+                        const T own = a2[q][a].x + a2[q][a].y;
+                        v[a] = own;
+                        for (int o = 1; o < g[q]; ++o) v[a] += __shfl_sync(0xffffffffu, own, (lane + o * len[q]) & 31);
+                    }
+                    if (grp[q] != 0) continue;
+                    const T *tl = taylor + static_cast<size_t>(c) * kTaylor;
+                    const T y[3] = {-nt[q][0].x, -nt[q][1].x, -nt[q][2].x};
+                    put(j[q], v[0] + tl[0] + tl[3] * y[0] + tl[4] * y[1] + tl[5] * y[2],
+                        v[1] + tl[1] + tl[6] * y[0] + tl[7] * y[1] + tl[8] * y[2],
+                        v[2] + tl[2] + tl[9] * y[0] + tl[10] * y[1] + tl[11] * y[2]);
+                }
+            }
+        } else {
+            T tl[kTaylor];
+#pragma unroll
+            for (int k = 0; k < kTaylor; ++k) tl[k] = taylor[static_cast<size_t>(c) * kTaylor + k];
+            for (int j0 = b; j0 < e; j0 += 32 * kSoftTPL) {
+                const int nq = min(kSoftTPL, (e - j0 + 31) / 32);  // warp-uniform
+                T ty[kSoftTPL][3], acc[kSoftTPL][3];
+#pragma unroll
+                for (int q = 0; q < kSoftTPL; ++q) {
+                    ty[q][0] = ty[q][1] = ty[q][2] = T(0);
+                    acc[q][0] = acc[q][1] = acc[q][2] = T(0);
+                    const int j = j0 + 32 * q + lane;
+                    if (q < nq && j < e) rel_pos<T>(j, xs, n, ph, pl, cd, cc, ty[q]);
+                }
+                SRec<T> nxt;
+                if (nsrc > 0) stage<T>(mom, moct, list[w][lane], cc, nxt);
                 for (int b0 = 0; b0 < nsrc; b0 += 32) {
                     batch[w][lane] = nxt;
                     __syncwarp();
@@ -613,25 +675,19 @@ __global__ void __launch_bounds__(kSoftWarps * 32, GB_SOFT_MIN_BLOCKS) k_soft_ne
                     }
                     __syncwarp();
                 }
-            }
 #pragma unroll
-            for (int q = 0; q < kSoftTPL; ++q) {
-                const int j = j0 + 32 * q + lane;
-                if (kPhi && q < nq && j < e) {
-                    const T *y = ty[q];
-                    // far levels: the centre's value and gradient (the field: a = grad phi here)
-                    farphi[j] += static_cast<double>(acc[q][0] + tl[12] + tl[0] * y[0] + tl[1] * y[1] + tl[2] * y[2]);
-                } else if (q < nq && j < e) {
-                    const T *y = ty[q];
-                    const T ax = acc[q][0] + tl[0] + tl[3] * y[0] + tl[4] * y[1] + tl[5] * y[2];
-                    const T ay = acc[q][1] + tl[1] + tl[6] * y[0] + tl[7] * y[1] + tl[8] * y[2];
-                    const T az = acc[q][2] + tl[2] + tl[9] * y[0] + tl[10] * y[1] + tl[11] * y[2];
-                    if (corr) {  // kept apart; soften_apply folds it into the far field
-                        corr[j] = ax, corr[n + j] = ay, corr[2 * static_cast<size_t>(n) + j] = az;
-                    } else {
-                        far[j] = G * (far[j] + ax);
-                        far[n + j] = G * (far[n + j] + ay);
-                        far[2 * static_cast<size_t>(n) + j] = G * (far[2 * static_cast<size_t>(n) + j] + az);
+                for (int q = 0; q < kSoftTPL; ++q) {
+                    const int j = j0 + 32 * q + lane;
+                    if (kPhi && q < nq && j < e) {
+                        const T *y = ty[q];
+                        // far levels: the centre's value and gradient (the field: a = grad phi here)
+                        farphi[j] += static_cast<double>(acc[q][0] + tl[12] + tl[0] * y[0] + tl[1] * y[1] + tl[2] * y[2]);
+                    } else if (q < nq && j < e) {
+                        const T *y = ty[q];
+                        const T ax = acc[q][0] + tl[0] + tl[3] * y[0] + tl[4] * y[1] + tl[5] * y[2];
+                        const T ay = acc[q][1] + tl[1] + tl[6] * y[0] + tl[7] * y[1] + tl[8] * y[2];
+                        const T az = acc[q][2] + tl[2] + tl[9] * y[0] + tl[10] * y[1] + tl[11] * y[2];
+                        put(j, ax, ay, az);
                     }
                 }
             }
@@ -648,20 +704,15 @@ __global__ void k_soft_apply(T *__restrict__ far, const T *__restrict__ corr, T 
         far[e] = G * (far[e] + corr[e]);
 }
 
-// corr: null writes far = G (far + correction) after L2P; non-null writes the
-// correction there (zeroed first), independent of the far-field chain.
+// Moments and leaf-centre terms.
 template <typename T>
-void launch_soften(Workspace &ws, T *corr) {
+void launch_soften_far(Workspace &ws) {
     const unsigned gw = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.c_cap, 4));  // a warp per leaf
     Mom<T> *mom = static_cast<Mom<T> *>(ws.smom);
     Mom<T> *moct = static_cast<Mom<T> *>(ws.smom_oct);
-    T *taylor = static_cast<T *>(ws.staylor);
-    const T e2 = static_cast<T>(ws.eps * ws.eps);
-    if (corr) cudaMemsetAsync(corr, 0, sizeof(T) * 3 * static_cast<size_t>(ws.n), ws.st);
     full_shared(k_mom_leaf<T>);
     full_shared(k_mom_up<T>);
     full_shared(k_soft_far<T>);
-    full_shared(k_soft_near<T>);
     k_mom_leaf<T><<<gw, 128, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_ctr, ws.xs, ws.ph,
                                          ws.pl, ws.n, ws.info, static_cast<T>(ws.m), mom, moct);
     ws.launches += 1;
@@ -671,11 +722,22 @@ void launch_soften(Workspace &ws, T *corr) {
         ws.launches += 1;
     }
     k_soft_far<T><<<gw, 128, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_level, ws.c_parent, ws.c_ctr, ws.info, ws.m2l_src,
-                                         mom, e2, taylor);
-    k_soft_near<T><<<gw, kSoftWarps * 32, 0, ws.st>>>(ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_parent,
-                                          ws.c_child, ws.c_ctr, ws.info, ws.m2l_src, mom, moct, taylor, ws.xs, ws.ph,
-                                          ws.pl, ws.n, e2, static_cast<T>(ws.G), static_cast<T *>(ws.farf), nullptr, corr);
-    ws.launches += 2;
+                                         mom, static_cast<T>(ws.eps * ws.eps), static_cast<T *>(ws.staylor));
+    ws.launches += 1;
+}
+
+// corr: null writes far = G (far + correction) after L2P; non-null writes the
+// correction there (zeroed first), independent of the far-field chain.
+template <typename T>
+void launch_soften_near(Workspace &ws, T *corr) {
+    const unsigned gw = capped_grid(static_cast<unsigned>(ws.num_sms) * 64, ceil_div(ws.c_cap, 4));  // a warp per leaf
+    if (corr) cudaMemsetAsync(corr, 0, sizeof(T) * 3 * static_cast<size_t>(ws.n), ws.st);
+    full_shared(k_soft_near<T>);
+    k_soft_near<T><<<gw, kSoftWarps * 32, 0, ws.st>>>(
+        ws.leaves, ws.d_counts, ws.c_begin, ws.c_end, ws.c_level, ws.c_parent, ws.c_child, ws.c_ctr, ws.info, ws.m2l_src,
+        static_cast<const Mom<T> *>(ws.smom), static_cast<const Mom<T> *>(ws.smom_oct), static_cast<const T *>(ws.staylor),
+        ws.xs, ws.ph, ws.pl, ws.n, static_cast<T>(ws.eps * ws.eps), static_cast<T>(ws.G), static_cast<T *>(ws.farf), nullptr, corr);
+    ws.launches += 1;
 }
 
 }  // namespace
@@ -707,20 +769,28 @@ size_t soften_cell_bytes(bool mixed) {
     return 16 * t;  // one Mom record
 }
 
+void soften_far(Workspace &ws) {
+    if (ws.mixed)
+        launch_soften_far<float>(ws);
+    else
+        launch_soften_far<double>(ws);
+}
+
 void soften_pass(Workspace &ws) {
     timer_begin(ws, kTSoft);
+    soften_far(ws);
     if (ws.mixed)
-        launch_soften<float>(ws, nullptr);
+        launch_soften_near<float>(ws, nullptr);
     else
-        launch_soften<double>(ws, nullptr);
+        launch_soften_near<double>(ws, nullptr);
     timer_end(ws, kTSoft);
 }
 
 void soften_corr(Workspace &ws) {
     if (ws.mixed)
-        launch_soften<float>(ws, static_cast<float *>(ws.soft_corr));
+        launch_soften_near<float>(ws, static_cast<float *>(ws.soft_corr));
     else
-        launch_soften<double>(ws, static_cast<double *>(ws.soft_corr));
+        launch_soften_near<double>(ws, static_cast<double *>(ws.soft_corr));
 }
 
 void soften_apply(Workspace &ws) {

@@ -241,7 +241,8 @@ int m2l_tc_row_floats(int p);
 const char *m2l_tc_encode(Workspace &ws);     // (re)build tmap_ms; nullptr or an error message
 void downward_pass(Workspace &ws);            // L2L + L2P into far
 void soften_pass(Workspace &ws);              // accurate mode: far = G (far + softening correction)
-void soften_corr(Workspace &ws);              // the same correction into soft_corr (no far-field input)
+void soften_far(Workspace &ws);               // its moments and leaf-centre terms
+void soften_corr(Workspace &ws);              // the rest of the correction, into soft_corr (no far-field input)
 void soften_apply(Workspace &ws);             // far = G (far + soft_corr)
 void soften_phi(Workspace &ws, double *farphi); // accurate mode: the far potential's correction (tree order)
 size_t soften_taylor_values();                // per-leaf values of the far levels' correction
