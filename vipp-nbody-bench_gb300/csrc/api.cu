@@ -465,8 +465,8 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
     // other), ms per step: 4M Plummer 30.4 and 32.9, 16M clustered 126.0 and 133.8,
     // 1M unit cube 5.7 and 6.3, 100,003 Plummer 3.00 and 3.40.
     const unsigned full = ws.p2p_blocks;
-    // FP64: four (57,344 of the registers at eight leave the M2L none): 16,384
-    // Plummer 4.53 and 4.83, 262,144 unit cube 27.5 and 28.2.
+    // FP64: four, whose 64 registers leave one M2L block its own: of two, three and
+    // four, 262,144 unit cube 23.9, 21.5 and 20.3 ms, 16,384 Plummer 4.53, 4.58 and 4.15.
     const unsigned beside = !ws.mixed ? 4u : ws.m2l_tensor ? 3u : 16u;
     const unsigned conc = std::min(ws.p2p_blocks_conc, beside);
     if (fork) {

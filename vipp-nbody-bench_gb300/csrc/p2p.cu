@@ -269,13 +269,22 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
     }
 }
 
-template <bool kSoft>
+// FP64: separations and factors from fixed-point positions (rinv.cuh pair_fixed), in a
+// frame per batch of 32 sources about the item's first target. Bound by the issue of
+// integer instructions (about 220 a pair; 3 FP64 operations hold the FP64 pipe for
+// 192 of its ~380 cycles). Per launch, with FP64 separations (6 FP64 operations,
+// 415 cycles): 131,071 Plummer 12.7 -> 10.4 ms, 262,144 unit cube 5.0 -> 4.2 ms; and the
+// FP64 pipe it leaves takes the M2L beside it: RK4 step of the cube 27.3 -> 20.4 ms.
+// 64 registers: builds of 72 to 96 are 3 to 8% faster alone, but leave the M2L
+// fewer registers beside four blocks (cube 21.5 to 24.5 ms). z's separation on the
+// FP64 pipe, as the direct sum has it: 4% faster alone, cube 22.4 ms.
 __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__restrict__ chunks, const unsigned *counts,
                                                             unsigned *queue, const LeafRec *__restrict__ recs,
                                                             const uint2 *__restrict__ ranges, const double *__restrict__ xs,
                                                             double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ nearv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
+    __shared__ int64_t fix[kP2PWarps][3][32];
     __shared__ double red[kP2PWarps][3][32], sum[kP2PWarps][3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
@@ -294,7 +303,13 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
         const int t = lane - grp * nt;
         const bool tact = grp < g;
         const int i = it.t0 + t;
-        const double tx = tact ? xs[i] : 0.0, ty = tact ? xs[n + i] : 0.0, tz = tact ? xs[2 * static_cast<size_t>(n) + i] : 0.0;
+        const double *ys = xs + n, *zs = ys + n;
+        // frames: extents of the item's targets and of a batch's sources about the first target
+        // (positions of targets are read again where they are needed: registers for them cost more)
+        const int r0 = it.t0;
+        const unsigned ttop = tact ? top_word(xs[i] - xs[r0], ys[i] - ys[r0], zs[i] - zs[r0]) : 0u;
+        int qf = INT_MIN;
+        int64_t gx = 0, gy = 0, gz = 0;
         sum[w][0][lane] = 0, sum[w][1][lane] = 0, sum[w][2][lane] = 0;  // the finished slices' sums
         for (int sl = it.sl; sl < it.se; ++sl) {
             unsigned v0, len;
@@ -304,22 +319,33 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
             cur.start(ranges + rec.x, rec.y, v0, len, static_cast<unsigned>(lane));
             unsigned j;
             for (unsigned cnt; (cnt = cur.next(static_cast<unsigned>(lane), j)) != 0;) {
+                double px = 0, py = 0, pz = 0;
+                unsigned top = ttop;
                 if (static_cast<unsigned>(lane) < cnt) {
-                    src[w][0][lane] = xs[j];
-                    src[w][1][lane] = xs[n + j];
-                    src[w][2][lane] = xs[2 * static_cast<size_t>(n) + j];
+                    px = xs[j], py = ys[j], pz = zs[j];
+                    src[w][0][lane] = px, src[w][1][lane] = py, src[w][2][lane] = pz;
+                    top = max(top, top_word(px - xs[r0], py - ys[r0], pz - zs[r0]));
+                }
+                const Frame fr = make_frame(static_cast<int>(__reduce_max_sync(0xffffffffu, top) >> 20), soft);
+                if (fr.ok) {
+                    fix[w][0][lane] = fixed_point(px, fr.qf), fix[w][1][lane] = fixed_point(py, fr.qf), fix[w][2][lane] = fixed_point(pz, fr.qf);
+                    if (fr.qf != qf) {
+                        qf = fr.qf;
+                        if (tact) gx = fixed_point(xs[i], qf), gy = fixed_point(ys[i], qf), gz = fixed_point(zs[i], qf);
+                    }
                 }
                 __syncwarp();
                 if (tact)
 #pragma unroll 2
                     for (unsigned k = grp; k < cnt; k += g) {
-                        const double dx = src[w][0][k] - tx, dy = src[w][1][k] - ty, dz = src[w][2][k] - tz;
-                        double f;
-                        if (!rinv3(dx, dy, dz, soft, f)) {
-                            const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                            double ri = rsqrt(r2);
-                            if (!kSoft) ri = r2 > 0.0 ? ri : 0.0;
-                            f = ri * ri * ri;
+                        double f, dx, dy, dz;
+                        if (!fr.ok || !pair_fixed(fix[w][0][k] - gx, fix[w][1][k] - gy, fix[w][2][k] - gz, soft, fr, f, dx, dy, dz)) {
+                            dx = src[w][0][k] - xs[i], dy = src[w][1][k] - ys[i], dz = src[w][2][k] - zs[i];
+                            if (dx == 0.0 && dy == 0.0 && dz == 0.0) continue;  // the target itself, or one at its place
+                            if (!rinv3(dx, dy, dz, soft, f)) {
+                                const double r2 = dx * dx + dy * dy + dz * dz + eps2, ri = r2 > 0.0 ? rsqrt(r2) : 0.0;
+                                f = ri * ri * ri;
+                            }
                         }
                         ax += f * dx;
                         ay += f * dy;
@@ -524,14 +550,9 @@ void p2p_pass(Workspace &ws, unsigned per_sm) {
         auto *o = static_cast<double *>(ws.nearf);
         auto *pd = static_cast<double *>(ws.part);
         const SoftInt si = soft_int(eps2);
-        full_shared(k_p2p_f64<true>);
-        full_shared(k_p2p_f64<false>);
-        if (soft)
-            k_p2p_f64<true><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges,
-                                                              ws.xs, pd, Gm, eps2, si, o, ws.n);
-        else
-            k_p2p_f64<false><<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges,
-                                                               ws.xs, pd, Gm, eps2, si, o, ws.n);
+        full_shared(k_p2p_f64);
+        k_p2p_f64<<<gs, kP2PWarps * 32, 0, ws.st>>>(ws.chunks, ws.d_counts, ws.queue, ws.leaf_rec, ws.ranges, ws.xs, pd, Gm, eps2,
+                                                    si, o, ws.n);
     }
     ws.launches += 1;
     timer_end(ws, kTP2P);

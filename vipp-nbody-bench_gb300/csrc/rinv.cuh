@@ -6,7 +6,7 @@
 // take 1-2. The sum of squares, the reciprocal root and its cube cost 12 of the
 // 18 FP64 operations of a softened pair; here they run on integers beside the
 // FP64 pipe, and a pair keeps 6 FP64 operations: the separation and the
-// accumulation (the same as before, in FP64).
+// accumulation; with the separation from fixed-point positions (Frame), 3.
 //
 // Arithmetic (fixed point, u = d^2 + eps^2):
 //   a_c   |d_c| as a 62-bit integer on a common exponent e (the largest of the
@@ -22,10 +22,10 @@
 // Exponents outside [-300, 300] (overflow, underflow, zero separation without
 // softening, infinities and NaN) are left to the FP64 form.
 //
-// Measured, FP64 operations 18 (or 36 with 1/sqrt) -> 6 (4) per pair: direct sum
-// of 4,096 targets over 262,144 sources 35.2 -> 11.7 ms (bound by the 6: 10.9
-// ms); near field of 131,071 Plummer particles (1.07e9 pairs) 39.6 -> 13.8 ms,
-// its potential 63 -> 8 ms; unit cube of 262,144 (4.0e8 pairs) 14.0 -> 5.0 ms.
+// Measured, FP64 operations per pair 18 (36 with 1/sqrt) -> 6 (4) -> 3 or 4 with
+// Frame: direct sum of 4,096 targets over 262,144 sources 35.2 -> 11.7 -> 8.2 ms; near
+// field of 131,071 Plummer particles (1.07e9 pairs) 39.6 -> 12.7 -> 10.4 ms, its
+// potential 63 -> 8 ms; unit cube of 262,144 (4.0e8 pairs) 14.0 -> 5.0 -> 4.2 ms.
 #pragma once
 
 #include <cstdint>
@@ -118,11 +118,7 @@ struct Root {
     int ef;         // common exponent field
 };
 
-GB_HD bool root(double dx, double dy, double dz, const SoftInt &e, Root &r) {
-    const uint32_t hx = hi_word(dx), hy = hi_word(dy), hz = hi_word(dz);
-    const int ef = max_field(max_field(static_cast<int>(hx & 0x7FF00000u), static_cast<int>(hy & 0x7FF00000u)),
-                             max_field(static_cast<int>(hz & 0x7FF00000u), e.ef));
-    const uint64_t ax = mantissa(hx, lo_word(dx), ef), ay = mantissa(hy, lo_word(dy), ef), az = mantissa(hz, lo_word(dz), ef);
+GB_HD void root_of(uint64_t ax, uint64_t ay, uint64_t az, int ef, const SoftInt &e, Root &r) {
     const uint32_t x1 = static_cast<uint32_t>(ax >> 32), y1 = static_cast<uint32_t>(ay >> 32), z1 = static_cast<uint32_t>(az >> 32);
     const uint64_t s2 = wide(x1, static_cast<uint32_t>(ax)) + wide(y1, static_cast<uint32_t>(ay)) + wide(z1, static_cast<uint32_t>(az));
     const uint64_t U = wide(x1, x1) + wide(y1, y1) + wide(z1, z1) + (s2 >> 31) +
@@ -142,6 +138,13 @@ GB_HD bool root(double dx, double dy, double dz, const SoftInt &e, Root &r) {
 #endif
     r.Y = Y, r.Q = Q, r.ef = ef;
     r.delta = static_cast<int>((static_cast<int64_t>(1ull << 56) - static_cast<int64_t>(prod) + 4) >> 3);
+}
+
+GB_HD bool root(double dx, double dy, double dz, const SoftInt &e, Root &r) {
+    const uint32_t hx = hi_word(dx), hy = hi_word(dy), hz = hi_word(dz);
+    const int ef = max_field(max_field(static_cast<int>(hx & 0x7FF00000u), static_cast<int>(hy & 0x7FF00000u)),
+                             max_field(static_cast<int>(hz & 0x7FF00000u), e.ef));
+    root_of(mantissa(hx, lo_word(dx), ef), mantissa(hy, lo_word(dy), ef), mantissa(hz, lo_word(dz), ef), ef, e, r);
     return ef >= kFieldLo && ef <= kFieldHi;
 }
 
@@ -153,10 +156,12 @@ GB_HD double pack(uint64_t m, int c, int ex) {
     const int lz = clz32(static_cast<uint32_t>(m >> 32)) - 1;  // top bit to bit 62
     m <<= lz;
     const int64_t corr = static_cast<int64_t>(static_cast<int32_t>(m >> 32)) * c;
-    uint64_t f = m + static_cast<uint64_t>(corr >> 21);
+    // 2^9: half a unit of the result where the correction does not carry m past a power of
+    // two (else up to a whole one); added before the last shift, after which it could pass 2^64
+    uint64_t f = m + static_cast<uint64_t>(corr >> 21) + 0x200;
     const int l2 = clz32(static_cast<uint32_t>(f >> 32));  // 0, 1 or 2
     f <<= l2;
-    return from_bits((static_cast<uint64_t>(1022 + 63 + ex - lz - l2) << 52) + ((f + 0x400) >> 11));
+    return from_bits((static_cast<uint64_t>(1022 + 63 + ex - lz - l2) << 52) + (f >> 11));
 }
 
 }  // namespace rinv
@@ -173,12 +178,18 @@ GB_HD SoftInt soft_int(double eps2) {
 }
 
 // false: outside the integer form's exponent range, the caller takes the FP64 form
+namespace rinv {
+GB_HD double cube(const Root &r) {
+    const uint64_t g = wide(static_cast<uint32_t>(r.Q >> 32), r.Y) + (wide(static_cast<uint32_t>(r.Q), r.Y) >> 32);
+    const int c = r.delta + (r.delta >> 1) + ((15 * square8(r.delta) + 32) >> 6);
+    return pack(g, c, -61 - 3 * ((r.ef >> 20) - 1023));
+}
+}  // namespace rinv
+
 GB_HD bool rinv3(double dx, double dy, double dz, const SoftInt &e, double &f) {
     rinv::Root r;
     const bool ok = rinv::root(dx, dy, dz, e, r);
-    const uint64_t g = rinv::wide(static_cast<uint32_t>(r.Q >> 32), r.Y) + (rinv::wide(static_cast<uint32_t>(r.Q), r.Y) >> 32);
-    const int c = r.delta + (r.delta >> 1) + ((15 * rinv::square8(r.delta) + 32) >> 6);
-    f = rinv::pack(g, c, -61 - 3 * ((r.ef >> 20) - 1023));
+    f = rinv::cube(r);
     return ok;
 }
 GB_HD bool rinv1(double dx, double dy, double dz, const SoftInt &e, double &f) {
@@ -187,6 +198,79 @@ GB_HD bool rinv1(double dx, double dy, double dz, const SoftInt &e, double &f) {
     const int c = (r.delta >> 1) + ((3 * rinv::square8(r.delta) + 32) >> 6);
     f = rinv::pack(static_cast<uint64_t>(r.Y) << 30, c, -61 - ((r.ef >> 20) - 1023));
     return ok;
+}
+
+// Separations as differences of fixed-point positions. A frame is a quantum 2^q for
+// a set of sources and targets whose separations stay below 2^(q+62): positions
+// as multiples of it modulo 2^64 (fixed_point), whose difference is the separation
+// whatever the positions' own size. Rounding a position costs half a quantum, so
+// separations of fewer than 53 bits of quanta are left to the FP64 difference: the
+// others are within 2^-53 of their largest component, as the FP64 difference is.
+struct Frame {
+    int ok;    // 0: no such frame (no extent, overflow, infinities, NaN, softening far above the extent)
+    int qf;    // exponent field of the quantum
+    int nmax;  // largest left shift of a separation that keeps eps below 2^62 quanta
+};
+// top: exponent field of the largest |component| of position - reference
+GB_HD Frame make_frame(int top, const SoftInt &e) {
+    const int ee = e.ef >> 20;
+    Frame f;
+    const int t = rinv::max_field(top, ee - 1);
+    f.qf = t - 60;
+    f.nmax = e.ef ? 61 - (ee - f.qf) : 62;
+    f.ok = top >= 1023 - 280 && t <= 1023 + 280 && t - top <= 2;
+    return f;
+}
+GB_HD uint64_t shl(uint64_t v, uint32_t s) {  // 0 from 64 on
+#ifdef __CUDA_ARCH__
+    uint64_t r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+    return r;
+#else
+    return s > 63 ? 0 : v << s;
+#endif
+}
+GB_HD int64_t fixed_point(double x, int qf) {  // x / 2^(qf - 1023) to the nearest, modulo 2^64
+    const uint32_t h = rinv::hi_word(x);
+    const int ex = static_cast<int>((h >> 20) & 0x7FFu);
+    const uint64_t m = ex ? (static_cast<uint64_t>((h & 0xFFFFFu) | 0x100000u) << 32) | rinv::lo_word(x) : 0;
+    const int s = ex - 52 - qf;  // m 2^s quanta
+    const uint64_t a = s >= 0 ? shl(m, static_cast<uint32_t>(s)) : (rinv::shr(m, static_cast<uint32_t>(-s - 1)) + 1) >> 1;
+    return static_cast<int64_t>((h >> 31) ? 0 - a : a);
+}
+namespace rinv {
+// a 2^(ef - 1023 - 61), a < 2^62, with the sign of s (0 or -1)
+GB_HD double to_double(uint64_t a, uint32_t s, int ef) {
+    const uint32_t h = static_cast<uint32_t>(a >> 32), l = static_cast<uint32_t>(a);
+    const uint64_t v = h ? a : static_cast<uint64_t>(l) << 31;
+    const uint32_t t = static_cast<uint32_t>(v >> 32);
+    const int lz = clz32(t) - 1;  // top bit to bit 62: the rounding cannot pass 2^64
+    const uint64_t m = v << (lz & 31);
+    const int field = (ef >> 20) - lz - (h ? 0 : 31);
+    const uint64_t b = (static_cast<uint64_t>(static_cast<uint32_t>(field)) << 52) + ((m + 0x200) >> 10);
+    return from_bits(t ? b | (static_cast<uint64_t>(s & 0x80000000u) << 32) : 0);
+}
+}  // namespace rinv
+
+// Separation (fx, fy, fz quanta of a frame that is ok) as doubles and its factor
+// f = (d^2 + eps^2)^(-3/2). false: too close for the frame, the caller takes the
+// FP64 difference of the positions.
+GB_HD bool pair_fixed(int64_t fx, int64_t fy, int64_t fz, const SoftInt &e, const Frame &fr, double &f, double &dx, double &dy,
+                      double &dz) {
+    const uint32_t sx = static_cast<uint32_t>(fx >> 63), sy = static_cast<uint32_t>(fy >> 63), sz = static_cast<uint32_t>(fz >> 63);
+    uint64_t ax = static_cast<uint64_t>(fx < 0 ? -fx : fx), ay = static_cast<uint64_t>(fy < 0 ? -fy : fy),
+             az = static_cast<uint64_t>(fz < 0 ? -fz : fz);
+    const uint32_t m = static_cast<uint32_t>(rinv::max_field(static_cast<int>(ax >> 32),
+                                                             rinv::max_field(static_cast<int>(ay >> 32), static_cast<int>(az >> 32))));
+    const int lead = rinv::clz32(m) - 2;  // 0 to 8 for the separations taken here
+    const int n = lead < fr.nmax ? lead : fr.nmax;
+    ax <<= n, ay <<= n, az <<= n;
+    const int ef = (fr.qf + 61 - n) << 20;
+    rinv::Root r;
+    rinv::root_of(ax, ay, az, ef, e, r);
+    f = rinv::cube(r);
+    dx = rinv::to_double(ax, sx, ef), dy = rinv::to_double(ay, sy, ef), dz = rinv::to_double(az, sz, ef);
+    return m >= (1u << 21);
 }
 
 }  // namespace gb
