@@ -38,8 +38,13 @@ constexpr int kDirectTB = 256;
 
 // Sources in tiles, each with its frame (rinv.cuh). Bound by the issue of integer
 // instructions (about 200 a pair, 4 FP64): 4,096 targets over 262,144 Plummer sources
-// 35.2 ms with the FP64 factor, 11.7 with the integer factor, 8.9 with the separations
-// from the frame, 8.2 with z's back on the FP64 pipe, which has room for it.
+// 35.2 ms with the FP64 factor, 11.7 with the integer factor, 9.2 with x's and y's
+// separations from the frame (z's stays on the FP64 pipe, which has room for it).
+// The frame of a tile is as wide as the system, so a few percent of the coordinates
+// are off its grid (rinv.cuh): x and y of a source off it, and those below 2^54 quanta to
+// a target off it (too_short), come from the FP64 pipe like z, one at a time. What is taken
+// is within 5/4 2^-53 of each component. The factor follows the pair's norm: off the grid
+// it is within 2^-50, as the FP64 form's.
 //
 // high word of the largest |component|: orders like the component; above 0x7FEFFFFF for infinities and NaN
 __device__ __forceinline__ unsigned top_word(double x, double y, double z) {
@@ -55,7 +60,7 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
                                                            double *__restrict__ part) {
     __shared__ double sx[kDirectTB], sy[kDirectTB], sz[kDirectTB], ref[3];
     __shared__ int64_t fx[kDirectTB], fy[kDirectTB], fz[kDirectTB];
-    __shared__ unsigned wtop[kDirectTB / 32];
+    __shared__ unsigned wtop[kDirectTB / 32], sgrid[kDirectTB / 32];
     const unsigned k = blockIdx.x * kDirectTB + threadIdx.x;
     bool act = k < nt;
     bool bad = false;
@@ -75,7 +80,7 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
     if (threadIdx.x == 0) ref[0] = tx, ref[1] = ty, ref[2] = tz;
     __syncthreads();
     const unsigned ttop = act ? top_word(tx - ref[0], ty - ref[1], tz - ref[2]) : 0u;
-    int qf = INT_MIN;
+    int qf = INT_MIN, kx = 0, ky = 0;
     int64_t gx = 0, gy = 0, gz = 0;
     for (unsigned b = lo; b < hi; b += kDirectTB) {
         const unsigned j = b + threadIdx.x;
@@ -95,16 +100,26 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
         const Frame fr = make_frame(static_cast<int>(top >> 20), soft);
         if (fr.ok) {
             fx[threadIdx.x] = fixed_point(px, fr.qf), fy[threadIdx.x] = fixed_point(py, fr.qf), fz[threadIdx.x] = fixed_point(pz, fr.qf);
-            if (fr.qf != qf)
+            if (fr.qf != qf) {
                 qf = fr.qf, gx = fixed_point(tx, qf), gy = fixed_point(ty, qf), gz = fixed_point(tz, qf);
+                kx = on_grid(tx, qf) ? 0 : kOffGrid, ky = on_grid(ty, qf) ? 0 : kOffGrid;
+            }
+            const unsigned g = __ballot_sync(0xffffffffu, on_grid(px, qf) && on_grid(py, qf));
+            if ((threadIdx.x & 31) == 0) sgrid[threadIdx.x >> 5] = g;
         }
         __syncthreads();
         const unsigned cnt = min(static_cast<unsigned>(kDirectTB), hi - b);
-        for (unsigned q = 0; q < cnt; ++q) {
+        unsigned grid = 0;
+        for (unsigned q = 0; q < cnt; ++q, grid >>= 1) {
+            if ((q & 31u) == 0) grid = sgrid[q >> 5];
             if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
             double f, dx, dy, unused;
             const double dz = sz[q] - tz;
-            if (!fr.ok || !pair_fixed(fx[q] - gx, fy[q] - gy, fz[q] - gz, soft, fr, f, dx, dy, unused)) {
+            const int64_t hx = fx[q] - gx, hy = fy[q] - gy;
+            if (fr.ok && pair_fixed(hx, hy, fz[q] - gz, soft, fr, f, dx, dy, unused)) {
+                if (!(grid & 1u) || too_short(hx, kx)) dx = sx[q] - tx;
+                if (!(grid & 1u) || too_short(hy, ky)) dy = sy[q] - ty;
+            } else {
                 dx = sx[q] - tx, dy = sy[q] - ty;
                 if (!rinv3(dx, dy, dz, soft, f)) {
                     const double ri = rsqrt(dx * dx + dy * dy + dz * dz + eps2);

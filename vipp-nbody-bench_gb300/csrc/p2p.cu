@@ -270,7 +270,11 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
 }
 
 // FP64: separations and factors from fixed-point positions (rinv.cuh pair_fixed), in a
-// frame per batch of 32 sources about the item's first target. Bound by the issue of
+// frame per batch of 32 sources about the item's first target. A pair takes them when
+// both positions are on the frame's grid, so that its separation is as exact in every
+// component as the FP64 difference, which the others take: a source off the grid alone,
+// and the whole batch where a target is off it (a tenth of a Plummer sphere's batches,
+// about the coordinate planes; none of a cube's inside). Bound by the issue of
 // integer instructions (about 220 a pair; 3 FP64 operations hold the FP64 pipe for
 // 192 of its ~380 cycles). Per launch, with FP64 separations (6 FP64 operations,
 // 415 cycles): 131,071 Plummer 12.7 -> 10.4 ms, 262,144 unit cube 5.0 -> 4.2 ms; and the
@@ -309,6 +313,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
         const int r0 = it.t0;
         const unsigned ttop = tact ? top_word(xs[i] - xs[r0], ys[i] - ys[r0], zs[i] - zs[r0]) : 0u;
         int qf = INT_MIN;
+        bool tgrid = false;  // every target of the item is on the grid of qf
         int64_t gx = 0, gy = 0, gz = 0;
         sum[w][0][lane] = 0, sum[w][1][lane] = 0, sum[w][2][lane] = 0;  // the finished slices' sums
         for (int sl = it.sl; sl < it.se; ++sl) {
@@ -327,19 +332,22 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
                     top = max(top, top_word(px - xs[r0], py - ys[r0], pz - zs[r0]));
                 }
                 const Frame fr = make_frame(static_cast<int>(__reduce_max_sync(0xffffffffu, top) >> 20), soft);
+                unsigned grid = 0;  // sources whose separations the frame holds exactly
                 if (fr.ok) {
                     fix[w][0][lane] = fixed_point(px, fr.qf), fix[w][1][lane] = fixed_point(py, fr.qf), fix[w][2][lane] = fixed_point(pz, fr.qf);
                     if (fr.qf != qf) {
                         qf = fr.qf;
                         if (tact) gx = fixed_point(xs[i], qf), gy = fixed_point(ys[i], qf), gz = fixed_point(zs[i], qf);
+                        tgrid = __all_sync(0xffffffffu, !tact || (on_grid(xs[i], qf) && on_grid(ys[i], qf) && on_grid(zs[i], qf)));
                     }
+                    grid = __ballot_sync(0xffffffffu, tgrid && on_grid(px, qf) && on_grid(py, qf) && on_grid(pz, qf));
                 }
                 __syncwarp();
                 if (tact)
 #pragma unroll 2
                     for (unsigned k = grp; k < cnt; k += g) {
                         double f, dx, dy, dz;
-                        if (!fr.ok || !pair_fixed(fix[w][0][k] - gx, fix[w][1][k] - gy, fix[w][2][k] - gz, soft, fr, f, dx, dy, dz)) {
+                        if (!(grid >> k & 1u) || !pair_fixed(fix[w][0][k] - gx, fix[w][1][k] - gy, fix[w][2][k] - gz, soft, fr, f, dx, dy, dz)) {
                             dx = src[w][0][k] - xs[i], dy = src[w][1][k] - ys[i], dz = src[w][2][k] - zs[i];
                             if (dx == 0.0 && dy == 0.0 && dz == 0.0) continue;  // the target itself, or one at its place
                             if (!rinv3(dx, dy, dz, soft, f)) {

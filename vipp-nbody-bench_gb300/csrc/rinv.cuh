@@ -203,9 +203,13 @@ GB_HD bool rinv1(double dx, double dy, double dz, const SoftInt &e, double &f) {
 // Separations as differences of fixed-point positions. A frame is a quantum 2^q for
 // a set of sources and targets whose separations stay below 2^(q+62): positions
 // as multiples of it modulo 2^64 (fixed_point), whose difference is the separation
-// whatever the positions' own size. Rounding a position costs half a quantum, so
-// separations of fewer than 53 bits of quanta are left to the FP64 difference: the
-// others are within 2^-53 of their largest component, as the FP64 difference is.
+// whatever the positions' own size. A coordinate with no bits below the quantum (on_grid:
+// all but those within 2^-8 of the set's extent of the coordinate planes) is held
+// exactly, so that between two of them every component, however small beside the
+// others, is rounded once, to 53 bits of its own, as the FP64 difference is (within
+// 2^-53 of itself). A coordinate off the grid is held to half a quantum: what that is
+// of a component depends on the component, and the kernels say which they take.
+// Pairs with no component of 53 bits of quanta are left to the FP64 difference.
 struct Frame {
     int ok;    // 0: no such frame (no extent, overflow, infinities, NaN, softening far above the extent)
     int qf;    // exponent field of the quantum
@@ -238,6 +242,17 @@ GB_HD int64_t fixed_point(double x, int qf) {  // x / 2^(qf - 1023) to the neare
     const uint64_t a = s >= 0 ? shl(m, static_cast<uint32_t>(s)) : (rinv::shr(m, static_cast<uint32_t>(-s - 1)) + 1) >> 1;
     return static_cast<int64_t>((h >> 31) ? 0 - a : a);
 }
+// fixed_point(x, qf) is x: the mantissa's last bit is no smaller than the quantum
+GB_HD bool on_grid(double x, int qf) {
+    const uint32_t h = rinv::hi_word(x);
+    return static_cast<int>((h >> 20) & 0x7FFu) >= qf + 52 || ((h << 1) | rinv::lo_word(x)) == 0;
+}
+// Below 2^54 quanta to a position off the grid (`off`: kOffGrid, or 0 for one on it): half a
+// quantum is then more than a quarter of the rounding to 53 bits.
+constexpr int kOffGrid = 1 << 22;  // high word of 2^54 quanta
+GB_HD bool too_short(int64_t f, int off) {  // in [-off, off) 2^32 quanta
+    return static_cast<uint32_t>(static_cast<int>(f >> 32) + off) < 2u * static_cast<uint32_t>(off);
+}
 namespace rinv {
 // a 2^(ef - 1023 - 61), a < 2^62, with the sign of s (0 or -1)
 GB_HD double to_double(uint64_t a, uint32_t s, int ef) {
@@ -248,7 +263,7 @@ GB_HD double to_double(uint64_t a, uint32_t s, int ef) {
     const uint64_t m = v << (lz & 31);
     const int field = (ef >> 20) - lz - (h ? 0 : 31);
     const uint64_t b = (static_cast<uint64_t>(static_cast<uint32_t>(field)) << 52) + ((m + 0x200) >> 10);
-    return from_bits(t ? b | (static_cast<uint64_t>(s & 0x80000000u) << 32) : 0);
+    return from_bits(a ? b | (static_cast<uint64_t>(s & 0x80000000u) << 32) : 0);
 }
 }  // namespace rinv
 
