@@ -4,7 +4,8 @@
 //   near    pairs of two positions on the grid (the near field; the others take the FP64 difference)
 //   direct  sources on the grid, and components that are not too_short to the target (the direct sum)
 // the worst relative error of their factor in units of 2^-51 (on the grid) and 2^-50 (off it),
-// and how many pairs or components of each were taken and left.
+// and how many pairs or components of each were taken and left, and how many differences
+// have their positions on either side of a multiple of 2^63 quanta.
 #include <cstdio>
 #include <cstdlib>
 #include <random>
@@ -14,19 +15,19 @@
 int main(int argc, char **argv) {
     if (argc < 4) return 2;
     const int axis = std::atoi(argv[1]);
-    const double h = std::atof(argv[2]), offset = std::atof(argv[3]);
+    const double h = std::atof(argv[2]), offset = std::atof(argv[3]), extent = argc > 4 ? std::atof(argv[4]) : 1;
     const gb::SoftInt e = gb::soft_int(1e-4);
     std::mt19937_64 g(11);
     std::uniform_real_distribution<double> U(-1, 1);
     constexpr int kN = 96;
     double x[kN][3];
     long double near = 0, direct = 0, factor = 0;
-    long near_taken = 0, near_left = 0, direct_taken = 0, direct_left = 0;
+    long wraps = 0, near_taken = 0, near_left = 0, direct_taken = 0, direct_left = 0;
     for (int rep = 0; rep < 60; ++rep) {
         int top = 0;
         for (int i = 0; i < kN; ++i)
             for (int a = 0; a < 3; ++a) {
-                x[i][a] = (a == axis ? offset + h * U(g) : U(g)) * 0.91;  // full mantissas
+                x[i][a] = (a == axis ? offset + h * U(g) : extent * U(g)) * 0.91;  // full mantissas
                 const int ex = static_cast<int>((gb::rinv::hi_word(x[i][a] - x[0][a]) >> 20) & 0x7FFu);
                 if (ex > top) top = ex;
             }
@@ -38,8 +39,8 @@ int main(int argc, char **argv) {
                 int64_t q[3];
                 bool on[2][3];
                 for (int a = 0; a < 3; ++a) {
-                    q[a] = static_cast<int64_t>(static_cast<uint64_t>(gb::fixed_point(x[j][a], f.qf)) -
-                                                static_cast<uint64_t>(gb::fixed_point(x[i][a], f.qf)));
+                    q[a] = gb::separation(gb::fixed_point(x[j][a], f.qf), gb::fixed_point(x[i][a], f.qf));
+                    wraps += (gb::fixed_point(x[j][a], f.qf) >> 63) != (gb::fixed_point(x[i][a], f.qf) >> 63);
                     on[0][a] = gb::on_grid(x[i][a], f.qf), on[1][a] = gb::on_grid(x[j][a], f.qf);
                 }
                 double fac, s[3];
@@ -64,7 +65,7 @@ int main(int argc, char **argv) {
                 factor = std::fmax(factor, std::fabs((fac - t * t * t) / (t * t * t)) * (both_on ? 0x1p51L : 0x1p50L));
             }
     }
-    std::printf("near %.4Lf direct %.4Lf factor %.4Lf near_taken %ld near_left %ld direct_taken %ld direct_left %ld\n", near, direct,
-                factor, near_taken, near_left, direct_taken, direct_left);
+    std::printf("near %.4Lf direct %.4Lf factor %.4Lf near_taken %ld near_left %ld direct_taken %ld direct_left %ld wraps %ld\n", near, direct,
+                factor, near_taken, near_left, direct_taken, direct_left, wraps);
     return 0;
 }

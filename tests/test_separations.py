@@ -18,7 +18,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 @pytest.fixture(scope="module")
 def exe(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("rinv") / "rinv_grid_check")
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", os.path.join(HERE, "rinv_grid_check.cpp"), "-o", out], check=True)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fsanitize=signed-integer-overflow,shift",
+                    "-fsanitize-undefined-trap-on-error", os.path.join(HERE, "rinv_grid_check.cpp"), "-o", out], check=True)
     return out
 
 
@@ -32,6 +33,16 @@ def test_components_against_long_double(exe, axis, h, offset):
     assert v["near"] <= 1.0 and v["direct"] <= 1.25 and v["factor"] <= 1.0
     if offset or h == 1.0:  # off the coordinate planes nearly every pair is taken
         assert v["near_taken"] > 20 * v["near_left"] and v["direct_taken"] > 20 * v["direct_left"]
+
+
+@pytest.mark.parametrize("offset", [0.5 / 0.91, 8 / 0.91, -8 / 0.91])
+def test_differences_wrap(exe, offset):
+    """Positions on both sides of a multiple of 2^63 quanta (an extent of 1/16 about 1/2, 8, -8): the build traps on
+    signed overflow, and the separations are as exact as elsewhere."""
+    r = subprocess.run([exe, "0", "0.06", repr(offset), "0.06"], capture_output=True, text=True, check=True)
+    f = r.stdout.split()
+    v = dict(zip(f[0::2], map(float, f[1::2])))
+    assert v["wraps"] > 50_000 and v["near"] <= 1.0 and v["direct"] <= 1.25 and v["factor"] <= 1.0
 
 
 @pytest.mark.gpu

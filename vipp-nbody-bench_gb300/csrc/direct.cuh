@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
                                                            unsigned nt, unsigned nsplit, double Gm, double eps2, SoftInt soft,
                                                            double *__restrict__ part) {
     __shared__ double sx[kDirectTB], sy[kDirectTB], sz[kDirectTB], ref[3];
-    __shared__ int64_t fx[kDirectTB], fy[kDirectTB], fz[kDirectTB];
+    __shared__ uint64_t fx[kDirectTB], fy[kDirectTB], fz[kDirectTB];
     __shared__ unsigned wtop[kDirectTB / 32], sgrid[kDirectTB / 32];
     const unsigned k = blockIdx.x * kDirectTB + threadIdx.x;
     bool act = k < nt;
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
     __syncthreads();
     const unsigned ttop = act ? top_word(tx - ref[0], ty - ref[1], tz - ref[2]) : 0u;
     int qf = INT_MIN, kx = 0, ky = 0;
-    int64_t gx = 0, gy = 0, gz = 0;
+    uint64_t gx = 0, gy = 0, gz = 0;
     for (unsigned b = lo; b < hi; b += kDirectTB) {
         const unsigned j = b + threadIdx.x;
         double px = 0, py = 0, pz = 0;
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
             if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
             double f, dx, dy, unused;
             const double dz = sz[q] - tz;
-            const int64_t hx = fx[q] - gx, hy = fy[q] - gy;
-            if (fr.ok && pair_fixed(hx, hy, fz[q] - gz, soft, fr, f, dx, dy, unused)) {
+            const int64_t hx = separation(fx[q], gx), hy = separation(fy[q], gy);
+            if (fr.ok && pair_fixed(hx, hy, separation(fz[q], gz), soft, fr, f, dx, dy, unused)) {
                 if (!(grid & 1u) || too_short(hx, kx)) dx = sx[q] - tx;
                 if (!(grid & 1u) || too_short(hy, ky)) dy = sy[q] - ty;
             } else {

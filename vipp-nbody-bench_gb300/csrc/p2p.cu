@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
                                                             double *__restrict__ part, double Gm, double eps2, SoftInt soft,
                                                             double *__restrict__ nearv, unsigned n) {
     __shared__ double src[kP2PWarps][3][32];
-    __shared__ int64_t fix[kP2PWarps][3][32];
+    __shared__ uint64_t fix[kP2PWarps][3][32];
     __shared__ double red[kP2PWarps][3][32], sum[kP2PWarps][3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned nch = counts[5];
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
         const unsigned ttop = tact ? top_word(xs[i] - xs[r0], ys[i] - ys[r0], zs[i] - zs[r0]) : 0u;
         int qf = INT_MIN;
         bool tgrid = false;  // every target of the item is on the grid of qf
-        int64_t gx = 0, gy = 0, gz = 0;
+        uint64_t gx = 0, gy = 0, gz = 0;
         sum[w][0][lane] = 0, sum[w][1][lane] = 0, sum[w][2][lane] = 0;  // the finished slices' sums
         for (int sl = it.sl; sl < it.se; ++sl) {
             unsigned v0, len;
@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
 #pragma unroll 2
                     for (unsigned k = grp; k < cnt; k += g) {
                         double f, dx, dy, dz;
-                        if (!(grid >> k & 1u) || !pair_fixed(fix[w][0][k] - gx, fix[w][1][k] - gy, fix[w][2][k] - gz, soft, fr, f, dx, dy, dz)) {
+                        if (!(grid >> k & 1u) || !pair_fixed(separation(fix[w][0][k], gx), separation(fix[w][1][k], gy),
+                                                             separation(fix[w][2][k], gz), soft, fr, f, dx, dy, dz)) {
                             dx = src[w][0][k] - xs[i], dy = src[w][1][k] - ys[i], dz = src[w][2][k] - zs[i];
                             if (dx == 0.0 && dy == 0.0 && dz == 0.0) continue;  // the target itself, or one at its place
                             if (!rinv3(dx, dy, dz, soft, f)) {

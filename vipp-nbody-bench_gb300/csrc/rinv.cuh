@@ -234,14 +234,18 @@ GB_HD uint64_t shl(uint64_t v, uint32_t s) {  // 0 from 64 on
     return s > 63 ? 0 : v << s;
 #endif
 }
-GB_HD int64_t fixed_point(double x, int qf) {  // x / 2^(qf - 1023) to the nearest, modulo 2^64
+GB_HD uint64_t fixed_point(double x, int qf) {  // x / 2^(qf - 1023) to the nearest, modulo 2^64
     const uint32_t h = rinv::hi_word(x);
     const int ex = static_cast<int>((h >> 20) & 0x7FFu);
     const uint64_t m = ex ? (static_cast<uint64_t>((h & 0xFFFFFu) | 0x100000u) << 32) | rinv::lo_word(x) : 0;
     const int s = ex - 52 - qf;  // m 2^s quanta
     const uint64_t a = s >= 0 ? shl(m, static_cast<uint32_t>(s)) : (rinv::shr(m, static_cast<uint32_t>(-s - 1)) + 1) >> 1;
-    return static_cast<int64_t>((h >> 31) ? 0 - a : a);
+    return (h >> 31) ? 0 - a : a;
 }
+// Source minus target in quanta. The positions are residues: their difference wraps in
+// ordinary runs (a leaf across x = 2^(q+63) has some on either side), so it is taken in
+// unsigned arithmetic and only the result, below 2^62 in size, is read with its sign.
+GB_HD int64_t separation(uint64_t source, uint64_t target) { return static_cast<int64_t>(source - target); }
 // fixed_point(x, qf) is x: the mantissa's last bit is no smaller than the quantum
 GB_HD bool on_grid(double x, int qf) {
     const uint32_t h = rinv::hi_word(x);
@@ -273,8 +277,8 @@ GB_HD double to_double(uint64_t a, uint32_t s, int ef) {
 GB_HD bool pair_fixed(int64_t fx, int64_t fy, int64_t fz, const SoftInt &e, const Frame &fr, double &f, double &dx, double &dy,
                       double &dz) {
     const uint32_t sx = static_cast<uint32_t>(fx >> 63), sy = static_cast<uint32_t>(fy >> 63), sz = static_cast<uint32_t>(fz >> 63);
-    uint64_t ax = static_cast<uint64_t>(fx < 0 ? -fx : fx), ay = static_cast<uint64_t>(fy < 0 ? -fy : fy),
-             az = static_cast<uint64_t>(fz < 0 ? -fz : fz);
+    const uint64_t ux = static_cast<uint64_t>(fx), uy = static_cast<uint64_t>(fy), uz = static_cast<uint64_t>(fz);
+    uint64_t ax = fx < 0 ? 0 - ux : ux, ay = fy < 0 ? 0 - uy : uy, az = fz < 0 ? 0 - uz : uz;
     const uint32_t m = static_cast<uint32_t>(rinv::max_field(static_cast<int>(ax >> 32),
                                                              rinv::max_field(static_cast<int>(ay >> 32), static_cast<int>(az >> 32))));
     const int lead = rinv::clz32(m) - 2;  // 0 to 8 for the separations taken here
