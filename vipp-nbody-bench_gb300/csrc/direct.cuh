@@ -113,8 +113,7 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
         for (unsigned q = 0; q < cnt; ++q, grid >>= 1) {
             if ((q & 31u) == 0) grid = sgrid[q >> 5];
             if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
-            double f, dx, dy, unused;
-            const double dz = sz[q] - tz;
+            double f, dx, dy, unused, dz = sz[q] - tz;
             const int64_t hx = separation(fx[q], gx), hy = separation(fy[q], gy);
             if (fr.ok && pair_fixed(hx, hy, separation(fz[q], gz), soft, fr, f, dx, dy, unused)) {
                 if (!(grid & 1u) || too_short(hx, kx)) dx = sx[q] - tx;
@@ -122,8 +121,10 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
             } else {
                 dx = sx[q] - tx, dy = sy[q] - ty;
                 if (!rinv3(dx, dy, dz, soft, f)) {
+                    // r^-3 leaves FP64's range at 1e103 and 1e-103, r^-2 (d / r) only with the result
                     const double ri = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
-                    f = ri * ri * ri;
+                    f = ri * ri;
+                    dx *= ri, dy *= ri, dz *= ri;
                 }
             }
             ax += f * dx;
