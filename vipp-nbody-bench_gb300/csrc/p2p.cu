@@ -109,7 +109,8 @@ template <bool kNewton, bool kSoft>
 __device__ __forceinline__ void pair2_f32(float2 x, float2 y, float2 z, float2 ntx, float2 nty, float2 ntz, float2 e2,
                                           float2 &ax, float2 &ay, float2 &az) {
     const float2 dx = __fadd2_rn(x, ntx), dy = __fadd2_rn(y, nty), dz = __fadd2_rn(z, ntz);
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+    float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+    if (kNewton) r2.x = fminf(r2.x, 3e38f), r2.y = fminf(r2.y, 3e38f);  // the step makes a NaN of infinity
     float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
     if (kNewton) {
         ri.x = ri.x * fmaf(-0.5f * r2.x * ri.x, ri.x, 1.5f);
@@ -122,9 +123,10 @@ __device__ __forceinline__ void pair2_f32(float2 x, float2 y, float2 z, float2 n
     az = __ffma2_rn(dz, f, az);
 }
 
-// Coordinate of the sources that fill up a slice's last batch: r^-3 of 1e18
-// underflows to 0, so they add exactly nothing.
-constexpr float kNowhere = 1e18f;
+// Coordinate of the sources that fill up a slice's last batch. r^2 overflows and its
+// reciprocal root is 0, so they add exactly nothing, whatever the system's size (1e18, where
+// r^-3 underflows, lay inside systems of that size).
+constexpr float kNowhere = 1e30f;
 
 // Compiled for 6 resident blocks per SM (80 registers). Bound by the FMA pipe
 // and what a batch costs beside its pairs: the pair loop alone reaches 8.9 pairs
