@@ -87,6 +87,8 @@ cudaError_t dalloc(T *&p, size_t count) {
     return cudaMalloc(reinterpret_cast<void **>(&p), sizeof(T) * count);
 }
 
+constexpr auto dalloc_fn = [](auto *&p, size_t count) { return dalloc(p, count); };
+
 void dfree(void *p) {
     if (p) cudaFree(p);
 }
@@ -284,22 +286,18 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
     if (!ws.mixed) {
         // class-group sums of the FP64 M2L's tiles while the tree is small
         const unsigned tiles = std::min(gb::kM2LSplitTiles, gb::m2l_f64_tiles(ws));
-        if (tiles > ws.m2l_part_tiles || ws.p > ws.m2l_part_p) {
+        if (!ws.f64_sums.holds(tiles, ws.p)) {
             ++ctx->epoch;
-            GB_TRY(dalloc(ws.m2l_part, gb::m2l_f64_part_doubles(ws.p) * tiles));
-            GB_TRY(dalloc(ws.m2l_pcnt, tiles));
-            GB_TRY(cudaMemsetAsync(ws.m2l_pcnt, 0, sizeof(unsigned) * tiles, ws.st));
-            ws.m2l_part_tiles = tiles, ws.m2l_part_p = ws.p;
+            GB_TRY(gb::resize(ws.f64_sums, tiles, ws.p, gb::m2l_f64_part_doubles(ws.p) * tiles, dalloc_fn));
+            GB_TRY(cudaMemsetAsync(ws.f64_sums.cnt, 0, sizeof(unsigned) * tiles, ws.st));
         }
     }
     if (ws.m2l_tensor) {
         // part sums of small trees' tiles (or a scratch per CTA)
         const unsigned tiles = std::min(gb::kM2LTcSplitTiles, gb::m2l_tc_tiles(ws));
-        if (tiles > ws.m2l_tc_tiles || ws.p > ws.m2l_tc_p) {
+        if (!ws.tc_sums.holds(tiles, ws.p)) {
             ++ctx->epoch;
-            GB_TRY(dalloc(ws.m2l_tc_part, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms))));
-            GB_TRY(dalloc(ws.m2l_tc_pcnt, tiles));
-            ws.m2l_tc_tiles = tiles, ws.m2l_tc_p = ws.p;
+            GB_TRY(gb::resize(ws.tc_sums, tiles, ws.p, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms)), dalloc_fn));
         }
         // split expansions of the tensor-core M2L and their TMA map
         const int kp = gb::m2l_tc_row_floats(ws.p);
@@ -538,6 +536,8 @@ int grow(gb_ctx *ctx, const unsigned *counts) {
 // Run f (which queues one or more evaluations) until no capacity overflow.
 template <typename F>
 int run_with_capacity(gb_ctx *ctx, F &&f) {
+    // its whole tiles fold their parts through the scratch at p >= 9
+    if (ctx->ws.n && ctx->ws.m2l_tensor && !ctx->ws.tc_sums.part) return ctx->err = "M2L scratch missing after a failed allocation", GB_ERR_CUDA;
     for (int attempt = 0; attempt < 6; ++attempt) {
         f();
         unsigned counts[gb::kNumCounts];
@@ -787,7 +787,7 @@ void gb_destroy(gb_ctx *ctx) {
                     ws.split_cell, ws.c_begin, ws.c_end, ws.c_parent, ws.c_child, ws.c_level, ws.c_path, ws.c_coord,
                     ws.c_box, ws.c_ctr, ws.Mexp, ws.Lexp, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                     ws.flag, ws.flag_off, ws.leaves, ws.rng_cnt, ws.rng_off, ws.leaf_rec, ws.ranges, ws.chunk_cnt,
-                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.m2l_tc_part, ws.m2l_tc_pcnt, ws.m2l_part, ws.m2l_pcnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
+                    ws.chunk_off, ws.chunks, ws.src_total, ws.part_cnt, ws.part_off, ws.part, ws.queue, ws.ops_d, ws.bimg, ws.m2l_tab, ws.ms_tc, ws.tc_sums.part, ws.tc_sums.cnt, ws.f64_sums.part, ws.f64_sums.cnt, ws.diag, ws.ops_f, ws.zf, ws.info, ws.d_counts, ctx->d_targets, ws.smom, ws.smom_oct, ws.staylor,
                     ctx->d_direct, ws.seg, ws.psys, ws.c_sys, ws.sys_par, ws.mkeys, ws.etile, ws.oct_list, ws.otile,
                     ws.ocnt, ws.soft_corr};
     for (void *b : bufs) dfree(b);

@@ -265,7 +265,7 @@ void launch_m2l_f64(Workspace &ws) {
     const unsigned gs = capped_grid(static_cast<unsigned>(ws.num_sms) * 2, static_cast<size_t>(m2l_f64_tiles(ws)) * kGroupsF64);
     k_m2l_f64<P><<<gs, kThreadsF64, smem, ws.st>>>(ws.info, ws.m2l_src, ws.ops_d, ws.forest() ? ws.otile : nullptr, ws.oct_list,
                                                    static_cast<const double *>(ws.Mexp), static_cast<double *>(ws.Lexp),
-                                                   ws.m2l_part, ws.m2l_pcnt, static_cast<int>(ws.m2l_part_tiles));
+                                                   ws.f64_sums.part, ws.f64_sums.cnt, static_cast<int>(ws.f64_sums.tiles));
     ws.launches += 1;
 }
 

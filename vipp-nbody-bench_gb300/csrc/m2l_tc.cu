@@ -762,8 +762,8 @@ void launch(Workspace &ws) {
     full_shared(k_split_m<P, BF>);
     full_shared(k_m2l_tc<P, BF>);
     k_split_m<P, BF><<<4 * ws.num_sms, 256, 0, ws.st>>>(ws.info, static_cast<const float *>(ws.Mexp), ws.ms_tc,
-                                                        static_cast<int>(ws.ms_rows), ws.m2l_tc_pcnt,
-                                                        static_cast<int>(ws.m2l_tc_tiles));
+                                                        static_cast<int>(ws.ms_rows), ws.tc_sums.cnt,
+                                                        static_cast<int>(ws.tc_sums.tiles));
     cudaFuncSetAttribute(k_m2l_tc<P, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C::SMEM));
     const unsigned ctas = std::max(1u, static_cast<unsigned>(ws.num_sms * ws.m2l_ctas_pct / 100));
     const unsigned gs = capped_grid(ctas, static_cast<size_t>(m2l_tc_tiles(ws)) * kParts);
@@ -771,7 +771,7 @@ void launch(Workspace &ws) {
                                                       reinterpret_cast<const unsigned char *>(ws.bimg),
                                                       forest ? ws.otile : nullptr, ws.oct_list,
                                                       static_cast<int>(ws.ms_rows), static_cast<float *>(ws.Lexp), ws.info,
-                                                      ws.m2l_tc_part, ws.m2l_tc_pcnt, static_cast<int>(ws.m2l_tc_tiles));
+                                                      ws.tc_sums.part, ws.tc_sums.cnt, static_cast<int>(ws.tc_sums.tiles));
     ws.launches += 2;
 }
 

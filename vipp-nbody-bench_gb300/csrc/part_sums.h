@@ -1,0 +1,30 @@
+// Scratch of an M2L whose tiles are shared out among work units (m2l_tc.cu,
+// m2l_fp64.cu): the units' partial sums and a counter per tile.
+#pragma once
+
+#include <cstddef>
+
+namespace gb {
+
+template <typename T>
+struct PartSums {
+    T *part = nullptr;
+    unsigned *cnt = nullptr;  // [tiles] finished units of a tile
+    unsigned tiles = 0;       // tiles the two are sized for
+    int p = 0;                // and the expansion order
+    bool holds(unsigned t, int q) const { return part && cnt && t <= tiles && q <= p; }
+};
+
+// Both buffers anew; alloc(pointer, count) frees what the pointer held, sets it (null
+// when it fails) and returns 0 or an error, which is passed on. Nothing is recorded as
+// held before both are there, so that after a failure no smaller request passes for met.
+template <typename T, class Alloc>
+auto resize(PartSums<T> &s, unsigned tiles, int p, std::size_t values, Alloc &&alloc) -> decltype(alloc(s.cnt, values)) {
+    s.tiles = 0, s.p = 0;
+    auto e = alloc(s.part, values);
+    if (e == decltype(e){}) e = alloc(s.cnt, static_cast<std::size_t>(tiles));
+    if (e == decltype(e){}) s.tiles = tiles, s.p = p;
+    return e;
+}
+
+}  // namespace gb

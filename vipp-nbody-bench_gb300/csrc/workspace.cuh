@@ -23,6 +23,7 @@
 
 #include "common.cuh"
 #include "harmonics.cuh"
+#include "part_sums.h"
 #include "prims.cuh"
 
 namespace gb {
@@ -165,14 +166,8 @@ struct Workspace {
     bool ms_bf16 = false;     // the split form tmap_ms was encoded for
     CUtensorMap tmap_ms{};    // TMA map of ms_tc
 
-    float *m2l_tc_part = nullptr;    // tensor-core M2L: part sums of small trees' tiles, or a scratch per CTA (m2l_tc.cu)
-    unsigned *m2l_tc_pcnt = nullptr; // [m2l_tc_tiles] finished parts of a tile (zeroed by k_split_m)
-    unsigned m2l_tc_tiles = 0;       // tiles the two are sized for
-    int m2l_tc_p = 0;                // and the expansion order
-    double *m2l_part = nullptr;   // FP64 M2L: class-group sums of small trees' tiles (m2l_fp64.cu)
-    unsigned *m2l_pcnt = nullptr; // [m2l_part_tiles] finished groups of a tile, zero between evaluations
-    unsigned m2l_part_tiles = 0;  // tiles the two are sized for
-    int m2l_part_p = 0;           // and the expansion order
+    PartSums<float> tc_sums;    // tensor-core M2L: part sums of small trees' tiles, or a scratch per CTA (counters zeroed by k_split_m)
+    PartSums<double> f64_sums;  // FP64 M2L: class-group sums of small trees' tiles (counters zero between evaluations)
 
     // device-side info and device-resident counters
     TreeInfo *info = nullptr;
