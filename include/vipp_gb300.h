@@ -286,7 +286,10 @@ GB_API int gb_direct_accel_noalloc(const double *x_dev, size_t n, const int64_t 
  * particle count, where the file has one. */
 typedef struct gb_tuning {
     int p2p_blocks;      /* P2P blocks per SM when the near field runs alone, 1..16 (default 8) */
-    int p2p_blocks_conc; /* P2P blocks per SM launched beside the far field, 0..16 (default 8) */
+    int p2p_blocks_conc; /* P2P blocks per SM launched beside the far field, 0..16. 8, the
+                            default: as many of 8 as the far field leaves room for (3 beside
+                            the tensor-core M2L, 4 in FP64); any other number is launched as
+                            it is (9 and more fill the SMs like 8) */
     int p2p_slice;       /* near-field sources per P2P work item, 1024..65536 (default 8192);
                             small systems take shorter ones (n / 32) */
     int m2l_ctas_pct;    /* tensor-core M2L CTAs, percent of the SMs, 10..100 (default 100) */

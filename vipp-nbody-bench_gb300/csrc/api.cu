@@ -51,7 +51,7 @@ struct gb_ctx {
     long long graph_steps = 0, direct_steps = 0, graph_captures = 0;
     std::vector<gb::PendingTimer> pending;
     std::vector<cudaEvent_t> free_events;
-    gb_tuning tune{8, 8, gb::kSliceSources, 100, 0, 0, 8};
+    gb_tuning tune{8, gb::kConcBlocksAuto, gb::kSliceSources, 100, 0, 0, 8};
     int tune_log2n = -1;  // size bucket the tuning cache was last applied for
     long long *d_targets = nullptr;
     size_t targets_cap = 0;
@@ -457,16 +457,16 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
     if (ws.forest()) gb::forest_tiles(ws, ws.m2l_tensor ? gb::kM2LTileTC : ws.mixed ? gb::kM2LTileCC : gb::kM2LTileF64);
     // Near field on the second stream, unless serial or timed: class timers
     // measure each class alone on one stream.
-    // Beside the far field, no more P2P blocks per SM than its tensor-core M2L leaves
-    // registers for (m2l_tc.cu): with more, the M2L's CTAs only
+    // Beside the far field, unless the tuning asks for another number, no more P2P blocks per
+    // SM than its tensor-core M2L leaves registers for (m2l_tc.cu): with more, the M2L's CTAs only
     // start when the near field is done. Three against eight (then one after the
     // other), ms per step: 4M Plummer 30.4 and 32.9, 16M clustered 126.0 and 133.8,
     // 1M unit cube 5.7 and 6.3, 100,003 Plummer 3.00 and 3.40.
     const unsigned full = ws.p2p_blocks;
     // FP64: four, whose 64 registers leave one M2L block its own: of two, three and
     // four, 262,144 unit cube 23.9, 21.5 and 20.3 ms, 16,384 Plummer 4.53, 4.58 and 4.15.
-    const unsigned beside = !ws.mixed ? 4u : ws.m2l_tensor ? 3u : 16u;
-    const unsigned conc = std::min(ws.p2p_blocks_conc, beside);
+    const unsigned beside = !ws.mixed ? 4u : ws.m2l_tensor ? 3u : gb::kConcBlocksAuto;
+    const unsigned conc = ws.p2p_blocks_conc == gb::kConcBlocksAuto ? beside : ws.p2p_blocks_conc;
     if (fork) {
         cudaEventRecord(ws.ev_fork, ws.st);
         cudaStreamWaitEvent(ws.st2, ws.ev_fork, 0);

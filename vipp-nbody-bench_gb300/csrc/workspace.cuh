@@ -42,6 +42,9 @@ struct alignas(16) LeafRec {
     float pad_;
 };
 
+// gb_tuning's p2p_blocks_conc by default: as many of 8 as the far field leaves room for
+constexpr int kConcBlocksAuto = 8;
+
 struct Workspace {
     // configuration of the evaluation
     int p = 4, K = 25, T = 90;  // T = floor(sqrt(8) s)
@@ -65,7 +68,7 @@ struct Workspace {
     int num_sms = 152;
     // tuning knobs (gb_set_tuning / the tuning cache; the defaults are the measured best at 4M)
     unsigned p2p_blocks = 8;        // P2P blocks per SM when it runs alone (or after the far field)
-    unsigned p2p_blocks_conc = 8;   // P2P blocks per SM launched beside the far field
+    unsigned p2p_blocks_conc = kConcBlocksAuto;  // P2P blocks per SM launched beside the far field
     unsigned p2p_slice = kSliceSources;  // near-field sources per P2P work item
     int m2l_ctas_pct = 100;         // tensor-core M2L CTAs, percent of the SMs (one persistent CTA per SM)
 

@@ -37,7 +37,7 @@ from . import MODE, PREC, TUNING_DEFAULT, TUNING_FIELDS, FLAG_M2L_BF16, Solver
 
 CANDIDATES = {
     "p2p_blocks": (4, 6, 8),
-    "p2p_blocks_conc": (0, 2, 4, 6, 8),
+    "p2p_blocks_conc": (0, 1, 2, 3, 4, 8),  # 8: the library's choice, 3 or 4
     "p2p_slice": (2048, 4096, 8192, 16384, 32768),
     "m2l_ctas_pct": (50, 75, 100),
     "serial": (0, 1),
