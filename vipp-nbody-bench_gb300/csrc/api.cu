@@ -285,7 +285,7 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
     }
     if (!ws.mixed) {
         // class-group sums of the FP64 M2L's tiles while the tree is small
-        const unsigned tiles = std::min(gb::kM2LSplitTiles, gb::m2l_f64_tiles(ws));
+        const unsigned tiles = std::min(gb::m2l_split_tiles(ws), gb::m2l_f64_tiles(ws));
         if (!ws.f64_sums.holds(tiles, ws.p)) {
             ++ctx->epoch;
             GB_TRY(gb::resize(ws.f64_sums, tiles, ws.p, gb::m2l_f64_part_doubles(ws.p) * tiles, dalloc_fn));
@@ -294,7 +294,7 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
     }
     if (ws.m2l_tensor) {
         // part sums of small trees' tiles (or a scratch per CTA)
-        const unsigned tiles = std::min(gb::kM2LTcSplitTiles, gb::m2l_tc_tiles(ws));
+        const unsigned tiles = std::min(gb::m2l_split_tiles(ws), gb::m2l_tc_tiles(ws));
         if (!ws.tc_sums.holds(tiles, ws.p)) {
             ++ctx->epoch;
             GB_TRY(gb::resize(ws.tc_sums, tiles, ws.p, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms)), dalloc_fn));

@@ -21,7 +21,7 @@
 // and no register tiling is needed.
 //
 // Small trees leave SMs idle with one block per 32 targets and octant, so
-// below kSplitTiles of them the 28 class groups of a tile run as blocks of their
+// up to m2l_split_tiles of them the 28 class groups of a tile run as blocks of their
 // own and the last one to finish adds the groups. Every form adds the groups in
 // the same order, so the results do not depend on it (a forest's systems keep
 // the bits of their own contexts).

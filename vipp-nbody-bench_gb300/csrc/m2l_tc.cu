@@ -53,7 +53,7 @@
 // three roles agree on it without exchanging control data.
 //
 // A tile's sum is made of six parts of 32 slots, each summed on its own and the
-// parts added in order. A tree of fewer than kSplitTiles tiles runs each part as
+// parts added in order. A tree of up to m2l_split_tiles tiles runs each part as
 // a work unit of its own (one CTA per tile would leave most SMs idle: 24 tiles at
 // 100,000 particles), leaves the part in a buffer and the CTA that finishes a
 // tile's last part adds the six; larger trees run whole tiles and fold the parts

@@ -205,12 +205,10 @@ constexpr int kM2LTileTC = 128;  // target octets per tensor-core M2L tile (m2l_
 constexpr int kZeroRows = 32;    // zero rows after the split expansions (one per row quad of a tile)
 constexpr int kM2LTileCC = 64;   // per FP32 CUDA-core M2L tile (fmm.cu)
 constexpr int kM2LTileF64 = 32;  // per FP64 M2L tile (m2l_fp64.cu)
-// Tensor-core M2L tiles up to which their parts run as units of their own: two
-// rounds of one CTA per SM (beyond that whole tiles fill the SMs)
-constexpr unsigned kM2LTcSplitTiles = 304;
-// FP64 M2L tiles (32 targets of one octant) up to which a tile's class groups
-// run as blocks of their own: two blocks on each of the 152 SMs
-constexpr unsigned kM2LSplitTiles = 304;
+// M2L tiles up to which a tile's parts (m2l_tc.cu) or class groups (m2l_fp64.cu) run as work
+// units of their own: two rounds of the tensor-core M2L's one CTA per SM, one of the
+// FP64 M2L's two blocks (beyond that whole tiles fill the SMs)
+inline unsigned m2l_split_tiles(const Workspace &ws) { return 2u * static_cast<unsigned>(ws.num_sms); }
 constexpr int kOpM2M = 343;  // op index of M2M octant 0
 constexpr int kOpL2L = 351;  // op index of L2L octant 0
 constexpr int kNumOps = 359;
