@@ -7,7 +7,13 @@
 
 #include "../vipp-nbody-bench_gb300/csrc/part_sums.h"
 
-int main() {
+int main(int argc, char **argv) {
+    if (argc == 7) {  // n, leaf, nsys, rows, bound, limit
+        unsigned long long v[6];
+        for (int i = 0; i < 6; ++i) v[i] = std::strtoull(argv[1 + i], nullptr, 10);
+        std::printf("%u\n", gb::split_tiles_held(v[0], v[1], v[2], static_cast<unsigned>(v[3]), static_cast<unsigned>(v[4]), static_cast<unsigned>(v[5])));
+        return 0;
+    }
     int fail_at = 0, calls = 0;
     auto alloc = [&](auto *&p, std::size_t count) {
         std::free(p);

@@ -201,6 +201,33 @@ int ensure_particles(gb_ctx *ctx, unsigned n) {
     return ensure_chunks(ctx);
 }
 
+// Scratch of the M2L's part sums for the cell buffers and the particles there are: up to
+// 120 MB (tensor cores) or 264 MB (FP64) at p = 10, 90 and 177 MB at p = 8 (there 7 and 28 MB
+// at 10,000 particles); at s = 64 the FP64 M2L has none from 1.8 million particles on and
+// the other its 7 MB from 7 million.
+int ensure_part_sums(gb_ctx *ctx) {
+    gb::Workspace &ws = ctx->ws;
+    auto held = [&](unsigned rows, unsigned bound) {
+        return gb::split_tiles_held(ws.n, static_cast<size_t>(ws.T), ws.forest() ? ws.nsys : 1, rows, bound, gb::m2l_split_tiles(ws));
+    };
+    if (!ws.mixed) {  // class-group sums of the FP64 M2L's tiles
+        const unsigned tiles = held(gb::kM2LTileF64, gb::m2l_f64_tiles(ws));
+        if (!ws.f64_sums.holds(tiles, ws.p)) {
+            ++ctx->epoch;
+            GB_TRY(gb::resize(ws.f64_sums, tiles, ws.p, gb::m2l_f64_part_doubles(ws.p) * tiles, dalloc_fn));
+            GB_TRY(cudaMemsetAsync(ws.f64_sums.cnt, 0, sizeof(unsigned) * tiles, ws.st));
+        }
+    }
+    if (ws.m2l_tensor) {  // part sums of tiles, or at least a scratch per CTA
+        const unsigned tiles = held(gb::kM2LTileTC, gb::m2l_tc_tiles(ws));
+        if (!ws.tc_sums.holds(tiles, ws.p)) {
+            ++ctx->epoch;
+            GB_TRY(gb::resize(ws.tc_sums, tiles, ws.p, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms)), dalloc_fn));
+        }
+    }
+    return GB_OK;
+}
+
 // Cell-indexed buffers for s_cap split cells (c_cap = 1 + 8 s_cap cells).
 int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
     gb::Workspace &ws = ctx->ws;
@@ -283,22 +310,9 @@ int ensure_cells(gb_ctx *ctx, unsigned s_cap, unsigned r_cap) {
         ws.soft_corr = c;
         ws.soft_corr_cap = ws.n_cap;
     }
-    if (!ws.mixed) {
-        // class-group sums of the FP64 M2L's tiles while the tree is small
-        const unsigned tiles = std::min(gb::m2l_split_tiles(ws), gb::m2l_f64_tiles(ws));
-        if (!ws.f64_sums.holds(tiles, ws.p)) {
-            ++ctx->epoch;
-            GB_TRY(gb::resize(ws.f64_sums, tiles, ws.p, gb::m2l_f64_part_doubles(ws.p) * tiles, dalloc_fn));
-            GB_TRY(cudaMemsetAsync(ws.f64_sums.cnt, 0, sizeof(unsigned) * tiles, ws.st));
-        }
-    }
+    const int rc = ensure_part_sums(ctx);
+    if (rc) return rc;
     if (ws.m2l_tensor) {
-        // part sums of small trees' tiles (or a scratch per CTA)
-        const unsigned tiles = std::min(gb::m2l_split_tiles(ws), gb::m2l_tc_tiles(ws));
-        if (!ws.tc_sums.holds(tiles, ws.p)) {
-            ++ctx->epoch;
-            GB_TRY(gb::resize(ws.tc_sums, tiles, ws.p, gb::m2l_tc_part_floats(ws.p, tiles, static_cast<unsigned>(ws.num_sms)), dalloc_fn));
-        }
         // split expansions of the tensor-core M2L and their TMA map
         const int kp = gb::m2l_tc_row_floats(ws.p);
         const unsigned rows = ws.c_cap + gb::kZeroRows;
@@ -555,7 +569,8 @@ int initial_capacity(gb_ctx *ctx) {
     gb::Workspace &ws = ctx->ws;
     const unsigned n = ws.n;
     const unsigned guess = 2 * (n / static_cast<unsigned>(ws.T + 1)) + 64;
-    if (ws.s_cap >= guess && ws.k_cap == ws.K * static_cast<int>(ws.mixed ? sizeof(float) : sizeof(double))) return GB_OK;
+    if (ws.s_cap >= guess && ws.k_cap == ws.K * static_cast<int>(ws.mixed ? sizeof(float) : sizeof(double)))
+        return ensure_part_sums(ctx);  // fewer particles than before may be a tree of few tiles
     return ensure_cells(ctx, std::max(guess, ws.s_cap), std::max(ws.r_cap, 32 * (1 + 8 * guess)));
 }
 

@@ -15,6 +15,15 @@ struct PartSums {
     bool holds(unsigned t, int q) const { return part && cnt && t <= tiles && q <= p; }
 };
 
+// Tiles the scratch has to hold: those of the cell buffers (`bound`), up to `limit`, beyond
+// which tiles run whole; none when no tree of these n particles can have as few as
+// `limit` tiles of `rows` targets (its leaves hold at most `leaf` particles each, and
+// at most 8 cells of each of the nsys trees are above level 2 and no targets).
+inline unsigned split_tiles_held(std::size_t n, std::size_t leaf, std::size_t nsys, unsigned rows, unsigned bound, unsigned limit) {
+    const std::size_t leaves = (n + leaf - 1) / leaf, targets = leaves > 8 * nsys ? leaves - 8 * nsys : 0;
+    return targets / rows > limit ? 0 : bound < limit ? bound : limit;
+}
+
 // Both buffers anew; alloc(pointer, count) frees what the pointer held, sets it (null
 // when it fails) and returns 0 or an error, which is passed on. Nothing is recorded as
 // held before both are there, so that after a failure no smaller request passes for met.
