@@ -791,12 +791,15 @@ __global__ void k_lists(const uint64_t *__restrict__ ent, const unsigned *counts
 // kLanes lanes per leaf, a lane per entry: a thread per leaf walked the ancestors'
 // lists entry by entry, a chain of ~100 dependent loads that took 30 us whatever the
 // tree's size (k_rng_fill; k_rng_count 11 to 15). A warp per leaf has the shortest
-// chain and is taken while one grid holds a warp for every leaf; beyond that the
-// instructions of idle lanes count, and 4 lanes are taken. Tree class per RK4 step,
+// chain and is taken up to 16 leaves per SM (two blocks of warps); beyond that the
+// instructions of idle lanes count, and 4 lanes are taken. The tree's own leaves decide,
+// on the device: the buffers may have been a larger system's. Tree class per RK4 step,
 // 4 / 8 / 16 / 32 lanes: 3,001 particles 0.519 / 0.497 / 0.485 / 0.482 ms; 100,003
 // 0.853 / 0.830 / 0.820 / 0.811; 4M 4.07 / 4.12 / 4.26 / 4.52; 16M 14.5 / 14.9 /
-// 15.5 / 16.6 (a thread per leaf: 0.62, 0.92, 4.03 and 14.7 or more).
-constexpr int kLeafLanesSmall = 32, kLeafLanesLarge = 4;
+// 15.5 / 16.6 (a thread per leaf: 0.62, 0.92, 4.03 and 14.7 or more). About the line, 4 / 32
+// lanes: Plummer of 995 leaves 0.770 / 0.731, 2,024 0.776 / 0.743, 3,767 0.818 / 0.803, 5,692
+// 0.943 / 0.940; cube of 3,571 0.673 / 0.679, of 4,096 0.778 / 0.797.
+constexpr int kLeafLanesSmall = 32, kLeafLanesLarge = 4, kWarpLeavesPerSM = 16;
 constexpr int kLeafBatch = 4;  // ranges a lane has in flight
 constexpr int kLeafThreads = 256;
 
@@ -834,13 +837,13 @@ __device__ __forceinline__ unsigned leaf_system_n(int c, unsigned n, const unsig
     return seg ? seg[c_sys[c] + 1] - seg[c_sys[c]] : n;
 }
 
+
 template <int kLanes>
-__global__ void __launch_bounds__(kLeafThreads) k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
+__device__ __forceinline__ void rng_count(int2 (*anc)[kMaxLevel + 1], const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
                             const int *__restrict__ c_begin, const int *__restrict__ c_end,
                             const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt, unsigned *rng_cnt,
                             unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, unsigned n,
                             const unsigned *__restrict__ seg, const int *__restrict__ c_sys) {
-    __shared__ int2 anc[kLeafThreads / kLanes][kMaxLevel + 1];
     const unsigned NL = counts[3];
     const int gl = threadIdx.x % kLanes, group = threadIdx.x / kLanes;
     constexpr unsigned kGroups = kLeafThreads / kLanes;
@@ -872,13 +875,27 @@ __global__ void __launch_bounds__(kLeafThreads) k_rng_count(const int *__restric
     }
 }
 
+__global__ void __launch_bounds__(kLeafThreads) k_rng_count(const int *__restrict__ leaves, const unsigned *counts, const int *__restrict__ c_parent,
+                            const int *__restrict__ c_begin, const int *__restrict__ c_end,
+                            const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt, unsigned *rng_cnt,
+                            unsigned *chunk_cnt, unsigned *src_total, unsigned *part_cnt, unsigned slice, unsigned n,
+                            const unsigned *__restrict__ seg, const int *__restrict__ c_sys, unsigned warp_leaves) {
+    __shared__ int2 anc[kLeafThreads / kLeafLanesLarge][kMaxLevel + 1];
+    if (counts[3] <= warp_leaves)
+        rng_count<kLeafLanesSmall>(anc, leaves, counts, c_parent, c_begin, c_end, p2p_own, p2p_cnt, rng_cnt, chunk_cnt, src_total,
+                                   part_cnt, slice, n, seg, c_sys);
+    else
+        rng_count<kLeafLanesLarge>(anc, leaves, counts, c_parent, c_begin, c_end, p2p_own, p2p_cnt, rng_cnt, chunk_cnt, src_total,
+                                   part_cnt, slice, n, seg, c_sys);
+}
+
 // Thread 0 first checks the near-field totals against the buffers: on any
 // overflow the evaluation queues no P2P work item at all (this kernel may still
 // address items whose partial-sum slot lies past part_cap, and the P2P kernels
 // run before the host sees the flag, grows the buffers and repeats the
 // evaluation).
 template <int kLanes>
-__global__ void __launch_bounds__(kLeafThreads) k_rng_fill(const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
+__device__ __forceinline__ void rng_fill(int2 (*anc)[kMaxLevel + 1], const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
                            const int *__restrict__ c_parent, const int *__restrict__ c_begin, const int *__restrict__ c_end,
                            const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt,
                            const unsigned *__restrict__ rng_off, LeafRec *leaf_rec, const double *__restrict__ c_ctr,
@@ -893,7 +910,6 @@ __global__ void __launch_bounds__(kLeafThreads) k_rng_fill(const int *__restrict
         counts[5] = over ? 0u : counts[5];
         info->n_p2p_chunks = static_cast<int>(counts[5]);
     }
-    __shared__ int2 anc[kLeafThreads / kLanes][kMaxLevel + 1];
     const unsigned NL = counts[3];
     constexpr unsigned kGroups = kLeafThreads / kLanes;
     constexpr unsigned kGroupMask = kLanes == 32 ? 0xffffffffu : (1u << (kLanes % 32)) - 1u;
@@ -975,6 +991,23 @@ __global__ void __launch_bounds__(kLeafThreads) k_rng_fill(const int *__restrict
         if (pairs) atomicAdd(reinterpret_cast<unsigned long long *>(&info->p2p_pairs), pairs);
         if (nranges) atomicAdd(reinterpret_cast<unsigned long long *>(&info->p2p_ranges), nranges);
     }
+}
+
+__global__ void __launch_bounds__(kLeafThreads) k_rng_fill(const int *__restrict__ leaves, unsigned *counts, unsigned r_cap, unsigned ch_cap,
+                           const int *__restrict__ c_parent, const int *__restrict__ c_begin, const int *__restrict__ c_end,
+                           const int *__restrict__ p2p_own, const int *__restrict__ p2p_cnt,
+                           const unsigned *__restrict__ rng_off, LeafRec *leaf_rec, const double *__restrict__ c_ctr,
+                           uint2 *ranges,
+                           const unsigned *__restrict__ chunk_off, int4 *chunks, const unsigned *__restrict__ src_total,
+                           const unsigned *__restrict__ part_off, unsigned part_cap, TreeInfo *info, unsigned slice, unsigned n,
+                           const unsigned *__restrict__ seg, const int *__restrict__ c_sys, unsigned warp_leaves) {
+    __shared__ int2 anc[kLeafThreads / kLeafLanesLarge][kMaxLevel + 1];
+    if (counts[3] <= warp_leaves)
+        rng_fill<kLeafLanesSmall>(anc, leaves, counts, r_cap, ch_cap, c_parent, c_begin, c_end, p2p_own, p2p_cnt, rng_off, leaf_rec,
+                                  c_ctr, ranges, chunk_off, chunks, src_total, part_off, part_cap, info, slice, n, seg, c_sys);
+    else
+        rng_fill<kLeafLanesLarge>(anc, leaves, counts, r_cap, ch_cap, c_parent, c_begin, c_end, p2p_own, p2p_cnt, rng_off, leaf_rec,
+                                  c_ctr, ranges, chunk_off, chunks, src_total, part_off, part_cap, info, slice, n, seg, c_sys);
 }
 
 // Start of an evaluation (one block): TreeInfo and the device counters zeroed,
@@ -1206,13 +1239,10 @@ void build_tree(Workspace &ws) {
     k_lists<<<gs, 256, 0, st>>>(ws.ent, ws.d_counts, ws.split_cell, ws.info, ws.c_child, ws.c_path, ws.c_coord,
                                 forest ? ws.c_sys : nullptr, ws.m2l_src, ws.p2p_own, ws.p2p_cnt, ws.coll, ws.coll_cnt,
                                 reinterpret_cast<unsigned long long *>(&ws.info->m2l_pairs));
-    // a warp per leaf while one grid has a warp for every leaf (figures at LeafEntries)
-    const unsigned full = static_cast<unsigned>(ws.num_sms) * 8;
-    const bool warp_each = ceil_div(ws.c_cap, kLeafThreads / kLeafLanesSmall) <= full;
-    const unsigned gl = warp_each ? ceil_div(ws.c_cap, kLeafThreads / kLeafLanesSmall)
-                                  : capped_grid(full, ceil_div(ws.c_cap, kLeafThreads / kLeafLanesLarge));
-    (warp_each ? k_rng_count<kLeafLanesSmall> : k_rng_count<kLeafLanesLarge>)<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
-        ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
+    const unsigned warp_leaves = static_cast<unsigned>(ws.num_sms) * kWarpLeavesPerSM;
+    const unsigned gl = capped_grid(static_cast<unsigned>(ws.num_sms) * 8, ceil_div(ws.c_cap, kLeafThreads / kLeafLanesSmall));
+    k_rng_count<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.c_parent, ws.c_begin, ws.c_end, ws.p2p_own, ws.p2p_cnt,
+        ws.rng_cnt, ws.chunk_cnt, ws.src_total, ws.part_cnt, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr, warp_leaves);
     {  // range, work-item and partial-slot offsets per leaf, one scan sequence
         ScanSet sc{};
         sc.in[0] = ws.rng_cnt, sc.out[0] = ws.rng_off, sc.total[0] = ws.d_counts + 4;
@@ -1220,9 +1250,9 @@ void build_tree(Workspace &ws) {
         sc.in[2] = ws.part_cnt, sc.out[2] = ws.part_off, sc.total[2] = ws.d_counts + 8;
         scan_exclusive_multi(sc, 3, ws.c_cap, ws.d_counts + 3, ws.scan, st, &ws.launches);
     }
-    (warp_each ? k_rng_fill<kLeafLanesSmall> : k_rng_fill<kLeafLanesLarge>)<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
+    k_rng_fill<<<gl, kLeafThreads, 0, st>>>(ws.leaves, ws.d_counts, ws.r_cap, ws.ch_cap, ws.c_parent, ws.c_begin, ws.c_end,
         ws.p2p_own, ws.p2p_cnt, ws.rng_off, ws.leaf_rec, ws.c_ctr, ws.ranges, ws.chunk_off, ws.chunks,
-        ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr);
+        ws.src_total, ws.part_off, ws.part_cap, ws.info, ws.p2p_slice, n, seg, forest ? ws.c_sys : nullptr, warp_leaves);
     ws.launches += 9;
     timer_end(ws, kTTree);
 }
