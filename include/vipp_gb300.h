@@ -397,7 +397,8 @@ GB_API int gb_tree_dump(gb_ctx *ctx, int64_t *ncells, int64_t *list_sizes, int32
                  int64_t *p2p_own, int64_t *coll_off, int64_t *coll);
 
 /* Kernel timing: when enabled, the context brackets each kernel class with
- * CUDA events on its stream and accumulates milliseconds and launch counts;
+ * CUDA events on its stream and accumulates milliseconds and how often the
+ * class ran (once per evaluation, in however many parts it is queued);
  * while it is on, the classes run one after another on one stream (no
  * near/far overlap) and every kernel is launched directly (no step graph).
  * Classes: 0 tree+lists, 1 operators, 2 P2M+M2M, 3 M2L, 4 L2L+L2P, 5 P2P,

@@ -26,6 +26,7 @@ void soa_to_aos(Workspace &ws, const double *soa, double *aos, unsigned n);
 
 struct PendingTimer {
     int cls;
+    bool more;  // a later part of the class's stage in the same evaluation
     cudaEvent_t a, b;
 };
 
@@ -337,7 +338,7 @@ void collect_timers(gb_ctx *ctx) {
         float ms = 0;
         if (cudaEventElapsedTime(&ms, pt.a, pt.b) == cudaSuccess) {
             ws.t_ms[pt.cls] += ms;
-            ws.t_launch[pt.cls] += 1;
+            ws.t_launch[pt.cls] += pt.more ? 0 : 1;
         }
         ctx->free_events.push_back(pt.a);
         ctx->free_events.push_back(pt.b);
@@ -356,7 +357,7 @@ const char *const kClassNames[gb::kNumTimers] = {"tree", "operators", "p2m_m2m",
 
 namespace gb {
 
-void timer_begin(Workspace &ws, int cls) {
+void timer_begin(Workspace &ws, int cls, bool more) {
     nvtx_push(kClassNames[cls]);
     if (!ws.timing || !g_timer_ctx) return;
     gb_ctx *ctx = g_timer_ctx;
@@ -370,7 +371,7 @@ void timer_begin(Workspace &ws, int cls) {
         }
         return e;
     };
-    PendingTimer pt{cls, take(), take()};
+    PendingTimer pt{cls, more, take(), take()};
     cudaEventRecord(pt.a, ws.st);
     ctx->pending.push_back(pt);
 }

@@ -1122,7 +1122,7 @@ void p2m_pass(Workspace &ws) {
 }
 
 void m2m_pass(Workspace &ws) {
-    timer_begin(ws, kTUp);
+    timer_begin(ws, kTUp, true);
     if (ws.mixed)
         dispatch_p<float>(ws, 3);
     else

@@ -863,7 +863,7 @@ void m2l_tc_images(Workspace &ws) {
 }
 
 void m2l_pass_tc(Workspace &ws) {
-    timer_begin(ws, kTM2L);
+    timer_begin(ws, kTM2L, true);
     launch_p(ws, false);
     timer_end(ws, kTM2L);
 }

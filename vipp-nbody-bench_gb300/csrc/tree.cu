@@ -1167,7 +1167,7 @@ void tree_box(Workspace &ws) {
 void build_tree(Workspace &ws) {
     const unsigned n = ws.n;
     cudaStream_t st = ws.st;
-    timer_begin(ws, kTTree);
+    timer_begin(ws, kTTree, true);
     const bool forest = ws.forest();
     if (!forest) {
         const int kbit = 3 * (kMaxLevel - ws.sort_levels);

@@ -278,7 +278,7 @@ inline void full_shared(F *kernel) {
 #endif
 
 // timing helpers
-void timer_begin(Workspace &ws, int cls);
+void timer_begin(Workspace &ws, int cls, bool more = false);  // more: another part of the class's stage, counted with the first
 void timer_end(Workspace &ws, int cls);
 
 #ifdef __CUDACC__
