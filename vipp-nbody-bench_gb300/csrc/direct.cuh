@@ -52,6 +52,11 @@ __device__ __forceinline__ unsigned top_word(double x, double y, double z) {
                max(static_cast<unsigned>(__double2hiint(y)) & 0x7FFFFFFFu, static_cast<unsigned>(__double2hiint(z)) & 0x7FFFFFFFu));
 }
 
+// dx = dy = dz = 0, off the FP64 pipe (three comparisons hold it as long as the three sums of a pair)
+__device__ __forceinline__ bool all_zero(double dx, double dy, double dz) {
+    return (top_word(dx, dy, dz) | static_cast<unsigned>(__double2loint(dx) | __double2loint(dy) | __double2loint(dz))) == 0;
+}
+
 // kCheckTargets: target indices come from device memory the host never saw;
 // an index outside [0, n) is not dereferenced and its result is NaN.
 template <class Pos, bool kCheckTargets = false>

@@ -29,7 +29,8 @@
 // Measured, ms per evaluation, a dense operator per source on tiles of 64 targets
 // -> this kernel: 217 cells, p = 4 2.04 -> 0.064; 745 cells, p = 4 3.57 -> 0.125;
 // 2,817 cells, p = 8 24.7 -> 2.38; 4,681 cells (unit cube), p = 6 10.3 -> 1.59.
-// Bound by the FP64 pipe (the operations above take 1.3 ms in the third case).
+// Bound by the FP64 pipe (the operations above take 1.3 ms in the third case; the pipe
+// is 87% active). 120 registers at p = 8; p = 10 spills 100 bytes at its 128.
 #include "workspace.cuh"
 
 namespace gb {

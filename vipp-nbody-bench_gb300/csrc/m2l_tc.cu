@@ -130,7 +130,8 @@ struct TcCfg {
     static constexpr int MMA_WARP = 4 + LOADERS;
     static constexpr int THREADS = 32 * (MMA_WARP + 1);
     // 64 registers, so that three P2P blocks (80 registers, one warp per scheduler
-    // each) fit beside this kernel's four warps on a scheduler
+    // each) fit beside this kernel's four warps on a scheduler (4 bytes spilled by the TF32
+    // builds of p = 5 and 10 and the BF16 build of p = 9)
     static constexpr int BOUND_THREADS = 512;
     static constexpr int BOUND_BLOCKS = 2;
     // Shared memory [coefficient][row]: the part's running sums where TMEM has no

@@ -135,7 +135,8 @@ constexpr float kNowhere = 1e30f;
 // a leaf's chunks fill 7.5; the kernel runs at 7.0 (4M Plummer, 1.03e10 pairs: 4.83
 // ms, 4.92 before; 1M unit cube 0.475 -> 0.465; 1M at p = 10 2.06 -> 1.96). A
 // 64-register build (8 blocks) spills 24 bytes and measured 1-5% slower on every
-// workload; a 96-register build kept the cluster M2M from starting beside P2P.
+// workload; a 96-register build kept the cluster M2M from starting beside P2P. The
+// softened kMulti build spills 8 bytes.
 // kMulti: items of several consecutive slices (a forest's); a single tree's items are
 // one slice each, and the bookkeeping between slices costs the kernel 1.7%.
 template <bool kNewton, bool kSoft, bool kMulti>
@@ -277,13 +278,13 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
 // component as the FP64 difference, which the others take: a source off the grid alone,
 // and the whole batch where a target is off it (a tenth of a Plummer sphere's batches,
 // about the coordinate planes; none of a cube's inside). Bound by the issue of
-// integer instructions (about 220 a pair; 3 FP64 operations hold the FP64 pipe for
-// 192 of its ~380 cycles). Per launch, with FP64 separations (6 FP64 operations,
-// 415 cycles): 131,071 Plummer 12.7 -> 10.4 ms, 262,144 unit cube 5.0 -> 4.2 ms; and the
-// FP64 pipe it leaves takes the M2L beside it: RK4 step of the cube 27.3 -> 20.4 ms.
-// 64 registers: builds of 72 to 96 are 3 to 8% faster alone, but leave the M2L
-// fewer registers beside four blocks (cube 21.5 to 24.5 ms). z's separation on the
-// FP64 pipe, as the direct sum has it: 4% faster alone, cube 22.4 ms.
+// integer instructions (about 220 a pair) and the FP64 pipe (3 operations a pair, 6 off
+// the grid, of 64 cycles each). Per launch, with FP64 separations throughout and as
+// built: 131,071 Plummer 13.2 and 10.5 ms, 262,144 unit cube 5.1 and 4.4 ms; and the
+// FP64 pipe it leaves takes the M2L beside it: RK4 step of the cube 28.3 and 21.1 ms.
+// 64 registers, 12 bytes spilled: builds of 72 to 96 are 1 to 8% faster alone, but leave
+// the M2L fewer registers beside four blocks (cube 24.6 to 25.9 ms). z's separation on
+// the FP64 pipe, as the direct sum has it: 4% faster alone, cube 22.4 ms.
 __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__restrict__ chunks, const unsigned *counts,
                                                             unsigned *queue, const LeafRec *__restrict__ recs,
                                                             const uint2 *__restrict__ ranges, const double *__restrict__ xs,
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 8) k_p2p_f64(const int4 *__res
                         if (!(grid >> k & 1u) || !pair_fixed(separation(fix[w][0][k], gx), separation(fix[w][1][k], gy),
                                                              separation(fix[w][2][k], gz), soft, fr, f, dx, dy, dz)) {
                             dx = src[w][0][k] - xs[i], dy = src[w][1][k] - ys[i], dz = src[w][2][k] - zs[i];
-                            if (dx == 0.0 && dy == 0.0 && dz == 0.0) continue;  // the target itself, or one at its place
+                            if (all_zero(dx, dy, dz)) continue;  // the target itself, or one at its place
                             if (!rinv3(dx, dy, dz, soft, f)) {
                                 const double r2 = dx * dx + dy * dy + dz * dz + eps2, ri = r2 > 0.0 ? rsqrt(r2) : 0.0;
                                 f = ri * ri * ri;

@@ -6,7 +6,8 @@
 // take 1-2. The sum of squares, the reciprocal root and its cube cost 12 of the
 // 18 FP64 operations of a softened pair; here they run on integers beside the
 // FP64 pipe, and a pair keeps 6 FP64 operations: the separation and the
-// accumulation; with the separation from fixed-point positions (Frame), 3.
+// accumulation; with the separation from fixed-point positions (Frame), 3 between
+// positions on its grid.
 //
 // Arithmetic (fixed point, u = d^2 + eps^2):
 //   a_c   |d_c| as a 62-bit integer on a common exponent e (the largest of the
@@ -23,9 +24,9 @@
 // softening, infinities and NaN) are left to the FP64 form.
 //
 // Measured, FP64 operations per pair 18 (36 with 1/sqrt) -> 6 (4) -> 3 or 4 with
-// Frame: direct sum of 4,096 targets over 262,144 sources 35.2 -> 11.7 -> 8.2 ms; near
-// field of 131,071 Plummer particles (1.07e9 pairs) 39.6 -> 12.7 -> 10.4 ms, its
-// potential 63 -> 8 ms; unit cube of 262,144 (4.0e8 pairs) 14.0 -> 5.0 -> 4.2 ms.
+// Frame: direct sum of 4,096 targets over 262,144 sources 35.2 -> 11.7 -> 9.2 ms; near
+// field of 131,071 Plummer particles (1.07e9 pairs) 39.6 -> 12.7 -> 10.5 ms, its
+// potential 63 -> 8 ms; unit cube of 262,144 (4.0e8 pairs) 14.0 -> 5.0 -> 4.4 ms.
 #pragma once
 
 #include <cstdint>
