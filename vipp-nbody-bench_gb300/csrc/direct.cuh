@@ -37,8 +37,8 @@ struct AoS {
 constexpr int kDirectTB = 256;
 
 // Sources in tiles, each with its frame (rinv.cuh). Bound by the issue of integer
-// instructions (about 200 a pair, 4 FP64): 4,096 targets over 262,144 Plummer sources
-// 35.2 ms with the FP64 factor, 11.7 with the integer factor, 9.2 with x's and y's
+// instructions (about 230 a pair, 4.2 FP64): 4,096 targets over 262,144 Plummer sources
+// 35.2 ms with the FP64 factor, 11.7 with the integer factor, 9.0 with x's and y's
 // separations from the frame (z's stays on the FP64 pipe, which has room for it).
 // The frame of a tile is as wide as the system, so a few percent of the coordinates
 // are off its grid (rinv.cuh): x and y of a source off it, and those below 2^54 quanta to
@@ -114,27 +114,30 @@ __global__ void __launch_bounds__(kDirectTB) k_direct_part(Pos pos, unsigned n, 
         }
         __syncthreads();
         const unsigned cnt = min(static_cast<unsigned>(kDirectTB), hi - b);
-        unsigned grid = 0;
-        for (unsigned q = 0; q < cnt; ++q, grid >>= 1) {
-            if ((q & 31u) == 0) grid = sgrid[q >> 5];
-            if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
-            double f, dx, dy, unused, dz = sz[q] - tz;
-            const int64_t hx = separation(fx[q], gx), hy = separation(fy[q], gy);
-            if (fr.ok && pair_fixed(hx, hy, separation(fz[q], gz), soft, fr, f, dx, dy, unused)) {
-                if (!(grid & 1u) || too_short(hx, kx)) dx = sx[q] - tx;
-                if (!(grid & 1u) || too_short(hy, ky)) dy = sy[q] - ty;
-            } else {
-                dx = sx[q] - tx, dy = sy[q] - ty;
-                if (!rinv3(dx, dy, dz, soft, f)) {
-                    // r^-3 leaves FP64's range at 1e103 and 1e-103, r^-2 (d / r) only with the result
-                    const double ri = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
-                    f = ri * ri;
-                    dx *= ri, dy *= ri, dz *= ri;
+        for (unsigned q0 = 0; q0 < cnt; q0 += 32) {
+            unsigned grid = sgrid[q0 >> 5];
+            const unsigned q1 = min(q0 + 32, cnt);
+#pragma unroll 1
+            for (unsigned q = q0; q < q1; ++q, grid >>= 1) {
+                if (b + q == i) continue;  // i == j is skipped (solver_ref_naive.hpp:109-111)
+                double f, dx, dy, unused, dz = sz[q] - tz;
+                const int64_t hx = separation(fx[q], gx), hy = separation(fy[q], gy);
+                if (fr.ok && pair_fixed(hx, hy, separation(fz[q], gz), soft, fr, f, dx, dy, unused)) {
+                    if (!(grid & 1u) || too_short(hx, kx)) dx = sx[q] - tx;
+                    if (!(grid & 1u) || too_short(hy, ky)) dy = sy[q] - ty;
+                } else {
+                    dx = sx[q] - tx, dy = sy[q] - ty;
+                    if (!rinv3(dx, dy, dz, soft, f)) {
+                        // r^-3 leaves FP64's range at 1e103 and 1e-103, r^-2 (d / r) only with the result
+                        const double ri = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
+                        f = ri * ri;
+                        dx *= ri, dy *= ri, dz *= ri;
+                    }
                 }
+                ax += f * dx;
+                ay += f * dy;
+                az += f * dz;
             }
-            ax += f * dx;
-            ay += f * dy;
-            az += f * dz;
         }
         __syncthreads();
     }

@@ -24,7 +24,7 @@
 // softening, infinities and NaN) are left to the FP64 form.
 //
 // Measured, FP64 operations per pair 18 (36 with 1/sqrt) -> 6 (4) -> 3 or 4 with
-// Frame: direct sum of 4,096 targets over 262,144 sources 35.2 -> 11.7 -> 9.2 ms; near
+// Frame: direct sum of 4,096 targets over 262,144 sources 35.2 -> 11.7 -> 9.0 ms; near
 // field of 131,071 Plummer particles (1.07e9 pairs) 39.6 -> 12.7 -> 10.5 ms, its
 // potential 63 -> 8 ms; unit cube of 262,144 (4.0e8 pairs) 14.0 -> 5.0 -> 4.4 ms.
 #pragma once
