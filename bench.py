@@ -92,7 +92,7 @@ def make_workload(args, rank=0, device=None):
 
 # DRAM bytes (read + write) per launch of the BF16-split M2L on the 4M
 # workload, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
-M2L_BF16_TRAFFIC = 135549184 + 14860544
+M2L_BF16_TRAFFIC = 135937024 + 17563392
 
 
 def batch_measure(steps=50, warmup=2, nsys=512, seed=3, sample=32, flags=0, form="forest", rank=0, ws=1, device=0):
@@ -401,8 +401,8 @@ def parse_args(argv=None):
                     help="ignore the library's tuning cache (vipp_gb300/tuning_gb300.txt): every line at the defaults")
     ap.add_argument("--tune-out", default=None, help="append the tuned entry to this tuning cache file")
     ap.add_argument("--p2p-occupancy", type=int, default=None, choices=[6, 8],
-                    help="override the tuning's mixed P2P kernel build for the main line (registers budgeted for "
-                         "8 or for 6 blocks per SM)")
+                    help="set the tuning's p2p_occupancy for the main line (accepted for old command lines: one build "
+                         "of the mixed P2P kernel serves both values)")
     ap.add_argument("--drift-steps", type=int, default=None,
                     help="untimed steps of the total-energy drift run (default: the 4M Plummer configuration's 100; 0 skips)")
     ap.add_argument("--acc-p", type=int, default=10, help="expansion order of the accurate-mode line")
@@ -621,7 +621,7 @@ def main():
         default_cfg = (args.workload == "plummer" and n == 1 << 22 and args.p == 8 and args.s == 64 and args.eps == 0.005
                        and args.precision == "mixed" and args.flags & ~vipp_gb300.FLAG_M2L_BF16 == 0)
         bf = bool(args.flags & vipp_gb300.FLAG_M2L_BF16)
-        traffic = {"p2p": 301173760 + 40833536, "m2l": (M2L_BF16_TRAFFIC if bf else 195950592 + 21233664)} if default_cfg else {}
+        traffic = {"p2p": 294412544 + 37558016, "m2l": (M2L_BF16_TRAFFIC if bf else 191850496 + 21219328)} if default_cfg else {}
         for k in per:
             per[k]["traffic"] = traffic.get(k)
         roof.update({"kernel": dom, "traffic": traffic.get(dom), "traffic_unit": "B per launch"})

@@ -478,8 +478,10 @@ void evaluate(gb_ctx *ctx, bool to_acc = true) {
     // other), ms per step: 4M Plummer 30.4 and 32.9, 16M clustered 126.0 and 133.8,
     // 1M unit cube 5.7 and 6.3, 100,003 Plummer 3.00 and 3.40.
     const unsigned full = ws.p2p_blocks;
-    // FP64: four, whose 64 registers leave one M2L block its own: of two, three and
-    // four, 262,144 unit cube 23.9, 21.5 and 20.3 ms, 16,384 Plummer 4.53, 4.58 and 4.15.
+    // FP64: four, whose 64 registers leave one M2L block its own. 2 / 3 / 4 / 8 and more, ms per
+    // step: 262,144 unit cube 25.2 / 26.0 / 20.9 / 24.6, 16,384 Plummer 4.85 / 4.86 / 4.39 / 4.14,
+    // 131,071 Plummer 55.7 / 54.0 / 58.0 / 52.8 (a Plummer sphere's M2L is a fifth of its near
+    // field and loses less by coming after it; p2p_blocks_conc = 16 asks for that).
     const unsigned beside = !ws.mixed ? 4u : ws.m2l_tensor ? 3u : gb::kConcBlocksAuto;
     const unsigned conc = ws.p2p_blocks_conc == gb::kConcBlocksAuto ? beside : ws.p2p_blocks_conc;
     if (fork) {

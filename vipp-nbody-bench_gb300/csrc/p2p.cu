@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(kP2PWarps * 32, 6) k_p2p_f32(const int4 *__res
 // frame per batch of 32 sources about the item's first target. A pair takes them when
 // both positions are on the frame's grid, so that its separation is as exact in every
 // component as the FP64 difference, which the others take: a source off the grid alone,
-// and the whole batch where a target is off it (a tenth of a Plummer sphere's batches,
-// about the coordinate planes; none of a cube's inside). Bound by the issue of
+// and the whole batch where a target is off it (together a quarter of the pairs of
+// 131,071 Plummer particles, about the coordinate planes; none inside a unit cube). Bound by the issue of
 // integer instructions (about 220 a pair) and the FP64 pipe (3 operations a pair, 6 off
 // the grid, of 64 cycles each). Per launch, with FP64 separations throughout and as
 // built: 131,071 Plummer 13.2 and 10.5 ms, 262,144 unit cube 5.1 and 4.4 ms; and the
